@@ -1,0 +1,47 @@
+"""Kernels at the sizes where their own tiling can go wrong, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BLOCK, STRIDE = 32768, 30720
+
+
+@pytest.mark.parametrize("system,mhz,insert", [("PAL", 40.0, 0), ("NTSC", 40.0, 0), ("NTSC", 20.0, 0),
+                                               ("NTSC", 93.0, 0), ("PAL", 40.0, 301), ("NTSC", 40.0, -257)])
+def test_float_tbc_matches_binary64(gpu, system, mhz, insert):
+    # the float TBC of the device's own streams and lines, luma and chroma in
+    # one pass, against the binary64 resampler: lines staged in shared memory
+    # at several sample rates, and (samples inserted or cut in mid-field) lines
+    # too long or too short for the stage.  The pair sums carry about 2^-46, so
+    # a float output differs only within 2^-22 of a rounding boundary; 1e-5 of
+    # the samples is 20 times that rate, and a uint16 then differs by 1.
+    from oracle import field, formats, sync, tbc
+    from vhsd_gb300 import native, synth
+    make = synth.pal_vhs if system == "PAL" else synth.ntsc_vhs
+    rf, info = synth.generate(make(fs=mhz * 1e6, fields=2, seed=3, snr_db=40.0))
+    if insert:
+        at = int(info["lead"] + 0.6 * info["field_samples"])
+        rf = np.concatenate([rf[:at], rf[at - insert:]])   # repeats `insert` samples, or cuts them
+    fmt = formats.get(system)
+    sp = sync.SyncParams(fmt, mhz * 1e6)
+    smoothing = fmt["sys"]["frame_lines"] / 2.0
+    nominal = float(round(fmt["sys"]["line_period"] * sp.mhz))
+    prof = native.PROFILE_PAL if system == "PAL" else native.PROFILE_NTSC
+    with native.Session(prof, len(rf), sample_rate_mhz=mhz) as s:
+        r = s.decode(rf, chroma=True)
+        assert r.fields >= 2
+        luma = s.tbc()
+        for i in range(r.fields):
+            fi = s.field(i)
+            length = r.stream_samples - fi.span_start
+            first = field.output_first_line(sp, bool(fi.is_first_field))
+            args = (s.lines(i), first, sp.output_lines, sp.outlinelen, nominal, smoothing)
+            hz = tbc.resample_field(s.stream(0, fi.span_start, length), *args)
+            want = tbc.to_u16(hz, sp, formats.output_scale(fmt), fmt["sys"]["outputZero"]).astype(np.int64)
+            diff = np.abs(luma[i].ravel().astype(np.int64) - want)
+            assert diff.max() <= 1 and np.mean(diff != 0) <= 1e-5, (i, diff.max(), np.mean(diff != 0))
+            want = tbc.resample_field(s.stream(3, fi.span_start, length), *args)
+            got = s.chroma_stage(i, 0)
+            assert np.mean(got != want) <= 1e-5, (i, np.mean(got != want))
+            assert np.max(np.abs(got - want)) <= 2.0 ** -23 * np.max(np.abs(want))

@@ -307,17 +307,21 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
     s->lut.alloc(lut.size());
     ck(cudaMemcpy(s->lut.p, lut.data(), lut.size() * sizeof(float), cudaMemcpyHostToDevice), "upload");
     {
-        // rows p and p+1 side by side: one 128-byte line per interpolated tap set
-        std::vector<float> pair((size_t)65536 * 32);
-        for (size_t r = 0; r < 65536; r++)
+        // rows p and p + 1 interleaved by groups of four taps: one 128-byte line
+        // per interpolated tap set, 32 bytes of it per four taps (the row after
+        // the last is the first, as the resampler wraps it)
+        std::vector<float> pair((size_t)65537 * 32);
+        for (size_t r = 0; r <= 65536; r++)
             for (int t = 0; t < 16; t++) {
-                pair[r * 32 + t] = lut[r * 16 + t];
-                pair[r * 32 + 16 + t] = lut[(r + 1) * 16 + t];
+                float* o = pair.data() + r * 32 + 8 * (t / 4) + t % 4;
+                o[0] = lut[r * 16 + t];
+                o[4] = lut[(r + 1) % 65537 * 16 + t];
             }
         s->lut_pair.alloc(pair.size());
         ck(cudaMemcpy(s->lut_pair.p, pair.data(), pair.size() * sizeof(float), cudaMemcpyHostToDevice),
            "upload");
     }
+    ck(prepare_tbc_kernels(), "tbc kernel attributes");
     double smoothing = s->fmt.frame_lines / 2.0;
     double alpha = 1.0 / (smoothing * s->outlen);
     std::vector<double> pw((size_t)s->outlen);

@@ -1279,13 +1279,148 @@ __global__ void k_tbc_consts(TbcParams p) {
     reinterpret_cast<TbcLineConsts*>(p.line_consts + t * kTbcLineConstsBytes)[0] = c;
 }
 
-constexpr int kTbcFastMaxThreads = 384;
-// kPair: a second source (src2 -> out2_f32) summed with the same taps; its own
-// instantiation, so the single-source kernel keeps its register count (two
-// CTAs per SM).
+constexpr int kTbcFastMaxThreads = 320;
+constexpr int kTbcStageBytes = 96 * 1024;   // most shared memory for a line's source
+constexpr int kTapRow = 16;   // floats of a sample's weight row
+// Where four taps 4 c .. 4 c + 3 of the warp's sample i lie in its row: both
+// the quads' stores and the lanes' loads of a row fill all 32 banks.
+__device__ __forceinline__ int tap_chunk(int i, int c) { return 4 * (c ^ ((i >> 1) & 3)); }
+
+// 16 consecutive floats of shared memory from at (4-byte aligned; up to three
+// floats before and after them are read too) with five 16-byte loads.
+__device__ __forceinline__ void load_taps(const float* at, float (&x)[16]) {
+    const uint32_t off = ((uint32_t)__cvta_generic_to_shared(at) >> 2) & 3u;
+    const float4* q = reinterpret_cast<const float4*>(at - off);
+    float v[20];
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const float4 u = q[i];
+        v[4 * i] = u.x; v[4 * i + 1] = u.y; v[4 * i + 2] = u.z; v[4 * i + 3] = u.w;
+    }
+    const bool two = (off & 2u) != 0, one = (off & 1u) != 0;
+#pragma unroll
+    for (int i = 0; i < 17; i++) v[i] = two ? v[i + 2] : v[i];
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = one ? v[i + 1] : v[i];
+}
+
+// Eight floats of the LUT (32-byte aligned).
+__device__ __forceinline__ void load_lut8(const float* p, float (&a)[4], float (&b)[4]) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3])
+        : "l"(p));
+}
+
+// Integer position, LUT row and interpolation weight of output sample k.
+struct TapPos {
+    int ci, ps;
+    float alpha;
+};
+__device__ __forceinline__ TapPos tap_pos(const TbcLineConsts& c, int k) {
+    const float2 kb = ff_mul((float)k, 0.0f, c.b.x, c.b.y);
+    const float2 pos = ff_add(c.a.x, c.a.y, kb.x, kb.y);
+    const float coord = __fadd_rn(pos.x, pos.y);
+    TapPos t;
+    t.ci = (int)coord;
+    const float pp = __fmul_rn(__fsub_rn(coord, (float)t.ci), 65536.0f);
+    t.ps = (int)pp;
+    t.alpha = __fsub_rn(pp, (float)t.ps);
+    t.ps = wrap_idx(t.ps, 65537);
+    return t;
+}
+
+// Packed pairs of floats (each half rounded as the scalar operation).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void two_sum(F2 a, F2 b, F2& s, F2& e) {
+    s = f2_add(a, b);
+    const F2 bb = f2_sub(s, a);
+    e = f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb));
+}
+
+// The sums of 16 float products (x w, and with kPair y w beside them in the
+// packed halves) as normalised float pairs (TwoSum), w read from shared memory
+// four at a time.  The products stay scalar: ptxas contracts a packed product
+// and a packed sum into a fused operation.
 template <bool kPair>
-__global__ void __launch_bounds__(kTbcFastMaxThreads) k_tbc_fast(const float* stream, int64_t stream_len,
-                                                                 TbcParams p) {
+__device__ __forceinline__ void tap_sums(const float (&x)[16], const float (&y)[16], const float* wrow, int lane,
+                                         float2& sx, float2& sy) {
+    if constexpr (kPair) {
+        F2 hi = 0, lo = 0;
+#pragma unroll
+        for (int t = 0; t < 16; t += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(wrow + tap_chunk(lane, t / 4));
+            const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                F2 s, e;
+                two_sum(hi, f2_pack(__fmul_rn(x[t + u], w[u]), __fmul_rn(y[t + u], w[u])), s, e);
+                hi = s;
+                lo = f2_add(lo, e);
+            }
+        }
+        F2 s, e;
+        two_sum(hi, lo, s, e);
+        const float2 h = f2_unpack(s), l = f2_unpack(e);
+        sx = make_float2(h.x, l.x);
+        sy = make_float2(h.y, l.y);
+    } else {
+        float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 16; t += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(wrow + tap_chunk(lane, t / 4));
+            const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                float s, e;
+                two_sum(hi, __fmul_rn(x[t + u], w[u]), s, e);
+                hi = s;
+                lo = __fadd_rn(lo, e);
+            }
+        }
+        two_sum(hi, lo, sx.x, sx.y);
+    }
+}
+
+// One CTA per output line, a lane per output sample.  What bounds it is the
+// shared-memory / L1 data path: 128 bytes of the sinc LUT at a random row and
+// 16 (with kPair 32) source floats per sample.  So:
+// * the line's stretch of the source is staged in shared memory once, and a
+//   lane reads its 16 floats with nine 8-byte loads (4 wavefronts a warp each;
+//   from global memory, 8 bytes a lane, 7);
+// * a warp fetches its 32 samples' LUT rows together, a quad of lanes per
+//   sample and 32 bytes a lane, so a row pair is one 128-byte access; the quad
+//   interpolates and leaves the 16 weights in the sample's shared row;
+// * each lane then sums its own sample alone, luma (and with kPair the chroma,
+//   src2 -> out2_f32, with the same weights) in packed pair additions.
+// Split over a quad, with a shuffled tree of pair additions per sample and
+// 4-byte source loads, the same sums cost 1000 instructions a luma and chroma
+// sample pair.
+template <bool kPair>
+__global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float* stream, int64_t stream_len,
+                                                                    TbcParams p, int stage_cap) {
+    extern __shared__ __align__(16) float tbc_smem[];
+    float* weights = tbc_smem;                                // [blockDim.x * kTapRow]
+    float* stage = weights + blockDim.x * kTapRow;            // [stage_cap], with kPair twice
     const int f = blockIdx.y;
     const int ol = blockIdx.x;
     const int64_t s0 = p.span_start[f];
@@ -1294,105 +1429,71 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads) k_tbc_fast(const float* st
     const float* src = stream + s0;
     const TbcLineConsts& c = *reinterpret_cast<const TbcLineConsts*>(
         p.line_consts + ((int64_t)f * p.out_lines + ol) * kTbcLineConstsBytes);
-    const float4* lut4 = reinterpret_cast<const float4*>(p.lut);
-    const float4* pair4 = reinterpret_cast<const float4*>(p.lut_pair);
     uint16_t* out = p.out_u16 ? p.out_u16 + ((int64_t)f * p.out_lines + ol) * p.outlen : nullptr;
     const float* src2 = p.src2 ? p.src2 + s0 : nullptr;
     float* out2 = p.out2_f32 ? p.out2_f32 + ((int64_t)f * p.out_lines + ol) * p.outlen : nullptr;
     float* outf32 = p.out_f32 ? p.out_f32 + ((int64_t)f * p.out_lines + ol) * p.out_stride - p.x0 : nullptr;
     const int kx1 = p.x1 > 0 ? p.x1 : p.outlen;
-    // Each lane owns one output sample (position, level and conversion done
-    // once); the 16-tap sums are gathered cooperatively: in round r the quad
-    // q of lanes works on the sample of lane 8 r + q, lane `sub` reading taps
-    // 4 sub .. 4 sub + 3, so a sample's 128-byte row pair is read by one
-    // quad in two coalesced accesses instead of eight scattered ones.
     const int lane = threadIdx.x & 31;
     const int q = lane >> 2, sub = lane & 3;
+    float* wrow = weights + (threadIdx.x & ~31) * kTapRow;   // the warp's 32 rows
+    // The stretch [lo, lo + len) of the span, four floats at a time, that the
+    // line's taps (positions run one way along the line) and load_taps's
+    // neighbours lie in.  A line whose taps leave the span or the stage (its
+    // locations are no line's) is read from global memory tap by tap.
+    const int first = tap_pos(c, p.x0).ci - 7, last = tap_pos(c, kx1 - 1).ci - 7;
+    const int lo = min(first, last) & ~3;
+    const int len = ((max(first, last) + 19 - lo) + 3) & ~3;
+    const bool staged = min(first, last) >= 0 && len > 0 && len <= stage_cap && lo + len <= n32;
+    if (staged) {
+        for (int i = 4 * threadIdx.x; i < len; i += 4 * blockDim.x) {
+            *reinterpret_cast<float4*>(stage + i) = __ldg(reinterpret_cast<const float4*>(src + lo + i));
+            if (kPair)
+                *reinterpret_cast<float4*>(stage + stage_cap + i) = __ldg(reinterpret_cast<const float4*>(src2 + lo + i));
+        }
+        __syncthreads();
+    }
     for (int k0 = p.x0; k0 < kx1; k0 += blockDim.x) {
         const int k = k0 + threadIdx.x;
         const bool valid = k < kx1;
-        const float kf = (float)(valid ? k : 0);
-        float2 kb = ff_mul(kf, 0.0f, c.b.x, c.b.y);
-        float2 pos = ff_add(c.a.x, c.a.y, kb.x, kb.y);
-        float coord = __fadd_rn(pos.x, pos.y);
-        int ci = (int)coord;
-        float fraction = __fsub_rn(coord, (float)ci);
-        float pp = __fmul_rn(fraction, 65536.0f);
-        int ps = (int)pp;
-        int pe = ps + 1;
-        float alpha = __fsub_rn(pp, (float)ps);
-        ps = wrap_idx(ps, 65537);
-        pe = wrap_idx(pe, 65537);
-        const int start = ci - 7;
-        const int interior = (n >= 16 && (uint32_t)start <= (uint32_t)(n - 16)) ? 1 : 0;
-        float hi_own = 0.0f, lo_own = 0.0f, hi2_own = 0.0f, lo2_own = 0.0f;
+        const TapPos tp = tap_pos(c, valid ? k : kx1 - 1);
+        // the warp's weights: in round r quad q fetches the row pair of the
+        // sample of lane 8 r + q, lane `sub` taps 4 sub .. 4 sub + 3
+        __syncwarp();   // the rows of the pass before have been read
 #pragma unroll
         for (int rnd = 0; rnd < 4; rnd++) {
             const int owner = rnd * 8 + q;
-            const int ps_o = __shfl_sync(0xffffffffu, ps, owner);
-            const int pe_o = __shfl_sync(0xffffffffu, pe, owner);
-            const int st_o = __shfl_sync(0xffffffffu, start, owner);
-            const float al_o = __shfl_sync(0xffffffffu, alpha, owner);
-            const int in_o = __shfl_sync(0xffffffffu, interior, owner);
-            float4 ws, we;
-            if (pe_o == ps_o + 1 && pair4) {
-                const float4* rs = pair4 + (int64_t)ps_o * 8;
-                ws = __ldg(rs + sub);
-                we = __ldg(rs + 4 + sub);
-            } else {
-                ws = __ldg(lut4 + (int64_t)ps_o * 4 + sub);
-                we = __ldg(lut4 + (int64_t)pe_o * 4 + sub);
-            }
-            const float wsv[4] = {ws.x, ws.y, ws.z, ws.w};
-            const float wev[4] = {we.x, we.y, we.z, we.w};
-            float hi = 0.0f, lo = 0.0f, hi2 = 0.0f, lo2 = 0.0f;
+            const int ps_o = __shfl_sync(0xffffffffu, tp.ps, owner);
+            const float al_o = __shfl_sync(0xffffffffu, tp.alpha, owner);
+            float ws[4], we[4];
+            load_lut8(p.lut_pair + ps_o * 32 + 8 * sub, ws, we);
+            float w[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                float wt = __fmaf_rn(al_o, __fsub_rn(wev[r], wsv[r]), wsv[r]);
+            for (int t = 0; t < 4; t++) w[t] = __fmaf_rn(al_o, __fsub_rn(we[t], ws[t]), ws[t]);
+            *reinterpret_cast<float4*>(wrow + owner * kTapRow + tap_chunk(owner, sub)) = make_float4(w[0], w[1], w[2], w[3]);
+        }
+        float x[16], x2[16];
+        const int start = tp.ci - 7;
+        if (staged) {
+            load_taps(stage + (start - lo), x);
+            if (kPair) load_taps(stage + stage_cap + (start - lo), x2);
+        } else {
+#pragma unroll
+            for (int t = 0; t < 16; t++) {
                 // 32-bit tap index: a field span is far below 2^31 samples
-                int idx = st_o + 4 * sub + r;
-                if (!in_o) {
+                int idx = start + t;
+                if (!(n >= 16 && (uint32_t)start <= (uint32_t)(n - 16))) {
                     if (idx < 0) idx += n32;
                     idx = idx < 0 ? 0 : (idx > n32 - 1 ? n32 - 1 : idx);
                 }
-                float prod = __fmul_rn(__ldg(src + idx), wt);
-                float s, e;
-                two_sum(hi, prod, s, e);
-                hi = s;
-                lo = __fadd_rn(lo, e);
-                if (kPair) {
-                    float prod2 = __fmul_rn(__ldg(src2 + idx), wt);
-                    two_sum(hi2, prod2, s, e);
-                    hi2 = s;
-                    lo2 = __fadd_rn(lo2, e);
-                }
-            }
-#pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
-                float oh = __shfl_xor_sync(0xffffffffu, hi, o);
-                float olo = __shfl_xor_sync(0xffffffffu, lo, o);
-                float2 t = ff_add(hi, lo, oh, olo);
-                hi = t.x;
-                lo = t.y;
-            }
-            // the owners of this round (lanes 8 rnd .. 8 rnd + 7) take their sums
-            const float rh = __shfl_sync(0xffffffffu, hi, 4 * (lane & 7));
-            const float rl = __shfl_sync(0xffffffffu, lo, 4 * (lane & 7));
-            if ((lane >> 3) == rnd) { hi_own = rh; lo_own = rl; }
-            if (kPair) {
-#pragma unroll
-                for (int o = 1; o < 4; o <<= 1) {
-                    float oh = __shfl_xor_sync(0xffffffffu, hi2, o);
-                    float olo = __shfl_xor_sync(0xffffffffu, lo2, o);
-                    float2 t = ff_add(hi2, lo2, oh, olo);
-                    hi2 = t.x;
-                    lo2 = t.y;
-                }
-                const float rh2 = __shfl_sync(0xffffffffu, hi2, 4 * (lane & 7));
-                const float rl2 = __shfl_sync(0xffffffffu, lo2, 4 * (lane & 7));
-                if ((lane >> 3) == rnd) { hi2_own = rh2; lo2_own = rl2; }
+                x[t] = __ldg(src + idx);
+                if (kPair) x2[t] = __ldg(src2 + idx);
             }
         }
+        __syncwarp();
+        float2 sum, sum2 = make_float2(0.0f, 0.0f);
+        tap_sums<kPair>(x, x2, wrow + lane * kTapRow, lane, sum, sum2);
+        const float hi_own = sum.x, lo_own = sum.y, hi2_own = sum2.x, lo2_own = sum2.y;
         if (!valid) continue;
         float2 la = c.adj;
         if (c.smooth) {
@@ -1432,6 +1533,13 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads) k_tbc_fast(const float* st
 }
 }  // namespace
 
+cudaError_t prepare_tbc_kernels() {
+    const int most = kTbcStageBytes + kTbcFastMaxThreads * kTapRow * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(k_tbc_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_tbc_fast<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // pw must hold (1-alpha)^(k+1) for k in [0, outlen) when smoothing > 0.
 // Float streams render with float-float accumulation when only uint16 output
 // is asked for; double streams and float-value outputs use binary64 as the
@@ -1447,15 +1555,21 @@ cudaError_t launch_tbc_pw(const T* stream, int64_t stream_len, const TbcParams& 
         p.line_consts) {
         const int64_t nl = (int64_t)p.nfields * p.out_lines;
         k_tbc_consts<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(p);
-        // a line in the fewest passes of at most 384 lanes, with the fewest idle
-        // lanes in the last pass (NTSC 910 samples: 3 x 320, PAL 1135: 3 x 384)
+        // a line in the fewest passes of at most 320 lanes (three CTAs of 64
+        // registers a lane), with the fewest idle lanes in the last pass (NTSC
+        // 910 samples: 3 x 320, PAL 1135: 4 x 288)
         const int width = (p.x1 > 0 ? p.x1 : p.outlen) - p.x0;
         const int passes = (width + kTbcFastMaxThreads - 1) / kTbcFastMaxThreads;
         const int threads = ((width + passes - 1) / passes + 31) / 32 * 32;
+        // the stage holds the window's stretch of a line 4 % longer than nominal
+        const int fit = ((int)(p.nominal * 1.04 * width / p.outlen) + 48) & ~3;
+        const int room = (kTbcStageBytes / (p.src2 ? 2 : 1) / (int)sizeof(float)) & ~3;
+        const int cap = fit < room ? fit : room;
+        const size_t smem = ((size_t)threads * kTapRow + (size_t)cap * (p.src2 ? 2 : 1)) * sizeof(float);
         if (p.src2)
-            k_tbc_fast<true><<<grid, threads, 0, s>>>(reinterpret_cast<const float*>(stream), stream_len, p);
+            k_tbc_fast<true><<<grid, threads, smem, s>>>(reinterpret_cast<const float*>(stream), stream_len, p, cap);
         else
-            k_tbc_fast<false><<<grid, threads, 0, s>>>(reinterpret_cast<const float*>(stream), stream_len, p);
+            k_tbc_fast<false><<<grid, threads, smem, s>>>(reinterpret_cast<const float*>(stream), stream_len, p, cap);
     } else {
         k_tbc<T><<<grid, 256, 0, s>>>(stream, stream_len, p, pw);
     }

@@ -181,7 +181,7 @@ struct TbcParams {
     double nominal;             // nominal input line length (samples)
     double smoothing;           // wow level-adjust smoothing (lines)
     const float* lut;           // [(65536+1)*16] sinc LUT
-    const float* lut_pair;      // optional [65536][32]: rows p and p+1 side by side
+    const float* lut_pair;      // [65536+1][4][2][4]: taps 4 s .. 4 s + 3 of rows p and p + 1 (65536: and 0)
     const float2* pw_ff;        // optional [outlen] pw as (hi, lo) float pairs
     double ire0, output_scale, inv_hz_ire, offset;  // uint16 conversion
     uint16_t* out_u16;          // [nfields * out_lines * outlen] or null
@@ -199,6 +199,8 @@ struct TbcParams {
 constexpr int kTbcLineConstsBytes = 64;
 constexpr int kTbcKernels = 2;      // levels + sinc (binary64 kernel)
 constexpr int kTbcFastKernels = 3;  // levels + line plans + sinc (float kernel)
+// Kernel attributes of the float kernel (once per device, outside any capture).
+cudaError_t prepare_tbc_kernels();
 // pw[k] = (1 - alpha)^(k+1), k < outlen, alpha = 1 / (smoothing * outlen)
 template <typename T>
 cudaError_t launch_tbc_pw(const T* video_stream, int64_t stream_len, const TbcParams& p,
