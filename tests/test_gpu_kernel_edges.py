@@ -45,3 +45,24 @@ def test_float_tbc_matches_binary64(gpu, system, mhz, insert):
             got = s.chroma_stage(i, 0)
             assert np.mean(got != want) <= 1e-5, (i, np.mean(got != want))
             assert np.max(np.abs(got - want)) <= 2.0 ** -23 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("nblocks,dtype", [(1, "int16"), (1, "float32"), (7, "float32"), (33, "int16"),
+                                           (800, "int16"), (801, "int16"), (865, "float32")])
+def test_chroma_block_stage_edges(gpu, nblocks, dtype):
+    # the block band-pass is bit-exact whatever the block's place in its CTA:
+    # one block, a part of a warp, one more than a CTA, and both sides of the
+    # line between 32 and 64 blocks a CTA (800 blocks); full-scale noise, so
+    # every sample of the odd extension and of the last chunk matters
+    from oracle import chroma, formats
+    from vhsd_gb300 import native
+    rng = np.random.default_rng(nblocks)
+    rf = rng.integers(-32768, 32768, (nblocks - 1) * STRIDE + BLOCK).astype(np.int16)
+    if dtype == "float32":
+        rf = (rf + rng.random(len(rf), np.float32)).astype(np.float32)
+    cp = chroma.ChromaParams(formats.get("NTSC"))
+    with native.Session(native.PROFILE_NTSC, len(rf)) as s:
+        s.decode(rf, demod_only=True, chroma=True)
+        for b in sorted({0, min(nblocks - 1, 31), min(nblocks - 1, 32), min(nblocks - 1, 64), nblocks - 1}):
+            want = chroma.chroma_stream(rf, cp, b, 1)
+            assert np.array_equal(s.stream(3, b * STRIDE, STRIDE), want), b

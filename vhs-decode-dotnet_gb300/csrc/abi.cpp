@@ -363,7 +363,9 @@ void ensure_chroma(vhsdecode_gb300_session* s) {
         throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "chroma band-pass pad length is not the block stage's");
     const size_t mf = (size_t)s->max_fields, field = (size_t)d.field_samples;
     const size_t win = (size_t)(2 * d.burst_end - d.burst_start);
-    s->c32.alloc((size_t)std::max<int64_t>(1, s->max_blocks) * kStride);
+    if (std::abs(d.move) > kCut)
+        throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "chroma offset rolls past the block cut");
+    s->c_mean.alloc((size_t)std::max<int64_t>(1, s->max_blocks));
     s->c_scratch.alloc((size_t)std::max<int64_t>(1, s->max_blocks) * kChromaRowStride);
     // Host fault injection, the counterpart of the reference build's forced
     // chroma-workspace failure (CUVHS_FORCE_CHROMA_WORKSPACE_FAILURE,
@@ -431,9 +433,7 @@ void ensure_chroma(vhsdecode_gb300_session* s) {
     s->chroma_alloc = true;
 }
 
-// The chroma channel of blocks [b0, b1) on stream `st` (the capture must be on
-// the device: rf16 or the session's float capture).
-void launch_chroma_blocks_for(vhsdecode_gb300_session* s, const int16_t* rf16, int64_t nblocks, cudaStream_t st) {
+ChromaBlockParams chroma_block_params(vhsdecode_gb300_session* s, const int16_t* rf16, int64_t nblocks) {
     ChromaBlockParams cb{};
     cb.rf16 = s->in_f32 ? nullptr : rf16;
     cb.rf32 = s->in_f32;
@@ -444,22 +444,54 @@ void launch_chroma_blocks_for(vhsdecode_gb300_session* s, const int16_t* rf16, i
     cb.c.edge = s->cd.rf.edge;
     cb.move = s->cd.move;
     cb.scratch = s->c_scratch.p;
-    cb.out = s->c32.p;
-    ck(launch_chroma_blocks(cb, st), "chroma block launch");
-    s->launches += kChromaBlockKernels;
+    cb.mean = s->c_mean.p;
+    return cb;
 }
 
-// The chroma block band-pass of the whole capture on the chroma stream, after
-// `after` (the point where the capture is on the device); the field batch
-// waits for chroma_done.  The kernel needs few SMs and is latency-bound, so it
-// runs beside the demodulator instead of after it.
+// The chroma block band-pass of the whole capture (on the device, or pinned
+// host memory that the device maps) on the chroma stream, after `after`.  It
+// holds few SMs and is latency-bound, so it runs beside the demodulator
+// instead of after it.
 void queue_chroma_blocks(vhsdecode_gb300_session* s, const int16_t* rf16, int64_t nblocks, cudaEvent_t after) {
     ck(cudaStreamWaitEvent(s->chroma_stream, after, 0), "wait");
     if (s->stage_timing) ck(cudaEventRecord(s->chroma_t[0], s->chroma_stream), "event");
-    launch_chroma_blocks_for(s, rf16, nblocks, s->chroma_stream);
+    ck(launch_chroma_blocks(chroma_block_params(s, rf16, nblocks), s->chroma_stream), "chroma block launch");
+    s->launches += kChromaBlockKernels;
     if (s->stage_timing) ck(cudaEventRecord(s->chroma_t[1], s->chroma_stream), "event");
+    s->chroma_blocks = nblocks;
+}
+
+// The blocks' means, after the band-pass and `after`; whoever reads the
+// channel waits for chroma_done.  They read every row again: after the field
+// analysis that runs beside the hsync kernels, which leave the memory idle,
+// instead of beside the demodulation.
+void queue_chroma_means(vhsdecode_gb300_session* s, cudaEvent_t after) {
+    if (s->chroma_blocks <= 0 || s->chroma_means) return;
+    ck(cudaStreamWaitEvent(s->chroma_stream, after, 0), "wait");
+    ck(launch_chroma_means(chroma_block_params(s, nullptr, s->chroma_blocks), s->chroma_stream), "chroma block launch");
     ck(cudaEventRecord(s->chroma_done, s->chroma_stream), "event");
-    s->chroma_pending = true;
+    s->chroma_means = true;
+}
+
+// The means of a decode whose field stage did not need them (no fields, or the
+// demodulation only), before `st` goes on.
+void finish_chroma_blocks(vhsdecode_gb300_session* s, cudaStream_t st) {
+    if (s->chroma_blocks <= 0 || s->chroma_means) return;
+    ck(cudaEventRecord(s->chroma_go, st), "event");
+    queue_chroma_means(s, s->chroma_go);
+    ck(cudaStreamWaitEvent(st, s->chroma_done, 0), "wait");
+}
+
+// The last decode's chroma channel, stitched into c32.
+void stitch_chroma(vhsdecode_gb300_session* s) {
+    if (s->c32_valid) return;
+    ck(cudaSetDevice(s->device), "cudaSetDevice");
+    const size_t want = (size_t)std::max<int64_t>(1, s->max_blocks) * kStride;
+    if (s->c32.n < want) s->c32.alloc(want);
+    ck(launch_chroma_stitch(chroma_block_params(s, nullptr, s->chroma_blocks), s->c32.p, s->chroma_stream),
+       "chroma stitch launch");
+    ck(cudaStreamSynchronize(s->chroma_stream), "sync");
+    s->c32_valid = true;
 }
 
 void session_free(vhsdecode_gb300_session* s) {
@@ -853,6 +885,10 @@ void launch_field_batch(vhsdecode_gb300_session* s, int f0, int f1, const T* vid
         ck(cudaEventRecord(s->drop_fork, fs), "event");
         ck(cudaStreamWaitEvent(ds, s->drop_fork, 0), "wait");
     }
+    if (chroma) {
+        if (timing) ck(cudaEventRecord(s->drop_fork, fs), "event");
+        queue_chroma_means(s, s->drop_fork);
+    }
     ck(launch_drop_mean<T>(env, stream_len, dp, s->drop_partial.p + (size_t)f0 * nch, ds), "dropout launch");
     HsyncParams hp{};
     hp.nfields = nf;
@@ -957,7 +993,12 @@ void launch_field_batch(vhsdecode_gb300_session* s, int f0, int f1, const T* vid
         ta.x0 = cp.win0;
         ta.x1 = cp.win0 + cp.win;
         ta.out_stride = cp.win;
-        ck(launch_tbc_pw<float>(s->c32.p, stream_len, ta, s->pw.p, fs), "chroma tbc launch");
+        ta.rows = s->c_scratch.p;
+        ta.row_mean = s->c_mean.p;
+        ta.row_offset = chroma_row_offset(d.move);
+        // the first reader of the chroma channel (the hsync kernels do not wait for it)
+        ck(cudaStreamWaitEvent(fs, s->chroma_done, 0), "wait");
+        ck(launch_tbc_pw<float>(nullptr, stream_len, ta, s->pw.p, fs), "chroma tbc launch");
         s->launches += kTbcFastKernels;
         ck(launch_chroma_phase(cp, fs), "chroma phase launch");
         s->launches += kChromaPhaseKernels;
@@ -983,7 +1024,9 @@ void launch_field_batch(vhsdecode_gb300_session* s, int f0, int f1, const T* vid
     const bool fused = chroma && std::is_same<T, float>::value;
     if (fused) {
         // the chroma TBC of the output lines rides on the luma's positions and weights
-        tp.src2 = s->c32.p;
+        tp.rows = s->c_scratch.p;
+        tp.row_mean = s->c_mean.p;
+        tp.row_offset = chroma_row_offset(s->cd.move);
         tp.out2_f32 = s->c_field.p + (size_t)f0 * s->cd.field_samples;
     }
     ck(launch_tbc_pw<T>(video, stream_len, tp, s->pw.p, fs), "tbc launch");
@@ -1000,7 +1043,10 @@ void launch_field_batch(vhsdecode_gb300_session* s, int f0, int f1, const T* vid
         tc.x1 = 0;
         tc.out_stride = s->outlen;
         tc.line_consts = s->tbc_consts.p + (size_t)f0 * s->out_lines * kTbcLineConstsBytes;
-        ck(launch_tbc_pw<float>(s->c32.p, stream_len, tc, s->pw.p, fs), "chroma tbc launch");
+        tc.rows = s->c_scratch.p;
+        tc.row_mean = s->c_mean.p;
+        tc.row_offset = chroma_row_offset(s->cd.move);
+        ck(launch_tbc_pw<float>(nullptr, stream_len, tc, s->pw.p, fs), "chroma tbc launch");
         s->launches += kTbcFastKernels;
         ck(launch_chroma_decode(cp, fs), "chroma decode launch");
         s->launches += kChromaDecodeKernels;
@@ -1086,7 +1132,7 @@ void collect_field_results(vhsdecode_gb300_session* s, cudaStream_t fs) {
         std::fprintf(stderr, "[gb300 stage] fields=%d hsync=%.3f ms tbc=%.3f ms dropouts=%.3f ms "
                      "rescue_fetches=%d enqueue=%.3f ms segments=%u porch_misses=%d\n", nf, s->stage_ms[0],
                      s->stage_ms[1], s->stage_ms[2], s->rescue_fetches, s->enqueue_ms, s->segments, miss);
-        if (s->chroma_pending) {
+        if (s->chroma_blocks > 0) {
             float c0 = 0, c1 = 0;
             ck(cudaEventSynchronize(s->chroma_t[1]), "sync");
             ck(cudaEventElapsedTime(&c0, s->ev[0], s->chroma_t[0]), "elapsed");
@@ -1220,7 +1266,6 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         cudaGetLastError();
     }
     if (carry && carry->no_graph) graphable = false;
-    s->chroma_pending = false;
     if (s->want_chroma && nblocks > 0 && host_input) {
         // The chroma block stage needs the whole capture and SMs of its own
         // for its whole run; queued behind the persistent demodulator it gets
@@ -1310,7 +1355,6 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         host_field_loop<float>(s, s->s32.p, stream_len, max_fields, feed, stop, cancel, carry);
         host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         ck(cudaEventRecord(s->ev[2], cs), "event");
-        if (s->chroma_pending) ck(cudaStreamWaitEvent(s->field_stream, s->chroma_done, 0), "wait");
         launch_field_batch<float>(s, 0, (int)s->fields.size(), s->v32.p, s->s32.p, s->e32.p,
                                   stream_len, s->field_stream);
         collect_field_results(s, s->field_stream);
@@ -1318,8 +1362,8 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         ck(cudaStreamWaitEvent(cs, s->field_end, 0), "wait");
     } else {
         ck(cudaEventRecord(s->ev[2], cs), "event");
-        if (s->chroma_pending) ck(cudaStreamWaitEvent(cs, s->chroma_done, 0), "wait");
     }
+    finish_chroma_blocks(s, cs);
     ck(cudaStreamSynchronize(s->d2h_stream), "sync");
     ck(cudaEventSynchronize(s->seg_dem[(size_t)(2 * std::max(0, nseg - 1) + 1)]), "sync");
     demod_ms = 0.0f;
@@ -1338,6 +1382,10 @@ void decode_plain(vhsdecode_gb300_session* s, const int16_t* rf_dev, uint64_t n,
     cudaStream_t cs = s->stream;
     int64_t nblocks = block_count(n);
     int64_t stream_len = nblocks * kStride;
+    if (s->want_chroma && nblocks > 0) {
+        ck(cudaEventRecord(s->chroma_go, cs), "event");
+        queue_chroma_blocks(s, rf_dev, nblocks, s->chroma_go);
+    }
     ck(cudaEventRecord(s->ev[1], cs), "event");
     run_demod(s, rf_dev, nblocks);
     s->launches += (uint32_t)(nblocks * (kPlainBlockKernels + (s->sub64.p ? kPlainSubKernels : 0)));
@@ -1363,12 +1411,10 @@ void decode_plain(vhsdecode_gb300_session* s, const int16_t* rf_dev, uint64_t n,
         auto t0 = std::chrono::steady_clock::now();
         host_field_loop<double>(s, s->s64.p, stream_len, max_fields, feed, stop, cancel, carry);
         host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        if (s->want_chroma) launch_chroma_blocks_for(s, rf_dev, nblocks, cs);
         launch_field_batch<double>(s, 0, (int)s->fields.size(), s->v64.p, s->s64.p, s->e64.p, stream_len, cs);
         collect_field_results(s, cs);
-    } else if (s->want_chroma && nblocks > 0) {
-        launch_chroma_blocks_for(s, rf_dev, nblocks, cs);
     }
+    finish_chroma_blocks(s, cs);
     ck(cudaEventSynchronize(s->ev[2]), "sync");
     ck(cudaEventElapsedTime(&demod_ms, s->ev[1], s->ev[2]), "elapsed");
 }
@@ -1430,6 +1476,8 @@ int32_t decode_impl(vhsdecode_gb300_session* s, const void* rf_in, uint64_t n_in
     const bool f32_in = (flags & VHSDECODE_GB300_DECODE_FLOAT_INPUT) != 0;
     s->want_chroma = (flags & VHSDECODE_GB300_DECODE_CHROMA) != 0;
     if (s->want_chroma) ensure_chroma(s);
+    s->chroma_blocks = 0;
+    s->chroma_means = s->c32_valid = false;
     if (!host_input && ((uintptr_t)rf_in & 15u) != 0)
         throw Failure(VHSDECODE_GB300_STATUS_INVALID_ARGUMENT, "device rf pointer must be 16-byte aligned");
     // samples at the decode rate
@@ -1893,6 +1941,7 @@ VHSDECODE_GB300_API int32_t VHSDECODE_GB300_CALL vhsdecode_gb300_session_copy_st
         ck(cudaStreamSynchronize(s->stream), "sync");
         if (channel == 3) {   // the chroma channel is float in both precisions
             std::vector<float> tmp(count);
+            stitch_chroma(s);
             ck(cudaMemcpy(tmp.data(), s->c32.p + start, count * sizeof(float), cudaMemcpyDeviceToHost), "d2h");
             for (uint64_t i = 0; i < count; i++) dst[i] = tmp[i];
         } else if (s->fp32()) {

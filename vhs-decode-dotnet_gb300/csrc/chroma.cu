@@ -9,7 +9,11 @@
 // operations, same order, one rounding each).
 // The roll by the chroma offset and the removal of the float mean
 // (ShiftChromaAndRemoveDcFloat32InPlace, VhsChromaDecoder.cs:2517-2533,
-// MeanFloat32FastMath :3751-3791) then stitch the block into the stream.
+// MeanFloat32FastMath :3751-3791) are left to the readers: the chroma channel
+// stays in the blocks' rows, with the blocks' means beside them, and the TBC
+// takes sample s of block b as row[b][s + offset] - mean[b].  (A stitched
+// stream cost a read and a write of every sample, 0.1 ms of a 41 M-sample
+// decode's demodulation; it is made when copy_stream asks for it.)
 //
 // Field stage: burst probes of the line-1 chroma TBC for both rotation
 // sequences of every field (ProbeUpconvertedBurstValue + DemodBurstFloat32,
@@ -82,20 +86,50 @@ struct LaneCascade {
 
 // ---------------------------------------------------------------- block stage
 
-// The block stage runs the 4-section cascade as a group of four lanes per
-// block, lane s running section s one 32-sample batch behind lane s - 1,
-// with its input fed from a ring of 32-sample chunks that cp.async fills
-// kRingDepth - 2 batches ahead (the latency of a global load is longer than
-// a batch of the recurrence), the lane-to-lane hand-over in registers
-// (shuffled as each output is made, consumed a batch later) and 16-byte stores
-// of the last section's outputs.
-constexpr int kExtBatches = kChromaExt / 32 + (kChromaExt % 32 != 0);
-constexpr int kRingDepth = 8;                       // chunks in flight per block
-constexpr int kRingSlot = 128;                      // bytes: 32 floats or 32 int16
-constexpr int kRingBytes = kRingDepth * kRingSlot + 16;   // + 16: blocks start on different banks
-constexpr int kBlockGroups = 64;                    // blocks per CTA (8 warps of 8 groups): two warps per
-                                                    // scheduler, so the stage holds few SMs beside the demod
+// The block stage.  Four lanes run a block's 4-section cascade, lane s section
+// s, 32 samples behind lane s - 1; a compute warp holds eight blocks.  What
+// bounds it is the recurrence: f -> c4 f -> (c1 v - c4 f) -> + z2 -> next f,
+// four dependent operations of 4.3 cycles a sample, 2 x 32,928 steps (0.55 ms).
+// A step is nine float operations, and all that is left around them in a
+// compute warp is 16-byte shared-memory accesses, the same for every lane: 16
+// inputs read a batch ahead, lane 0's from the input ring, the others' from
+// the ring their predecessor writes.  A helper warp per compute warp does the
+// rest in the issue slots the chain leaves free: cp.async of the source
+// several chunks (of 32 samples) ahead, the odd extension, the int16
+// conversion, the reversal for the backward pass, and the 16-byte stores of
+// lane 3's outputs.  The two meet at a barrier once per chunk.  Sample e is
+// taken at step e + 5, where the source, the rows and the chunks all fall on
+// 16-byte boundaries.
+constexpr int kExtBatches = kChromaExt / 32 + (kChromaExt % 32 != 0);   // chunks of the extended block
+constexpr int kIirLead = kChromaRowShift;           // step of the first sample
+constexpr int kIirLag = 32;                         // steps between neighbouring lanes
+constexpr int kIirChunks = (kChromaExt + kIirLead + 3 * kIirLag + 31) / 32;
+constexpr int kRawDepth = 16;                       // source chunks in flight or waiting (a capture read through
+                                                    // mapped host memory has the longest latency to cover)
+// Shared memory of a block: source chunks (128 bytes: 32 floats, or 32 int16
+// in the first 64), the input ring (4 chunks), the output ring (2 chunks),
+// lanes 0 .. 2's hand-over rings (two batches of 16 floats each); the rings
+// that the four lanes access together lie on different banks.
+constexpr int kIirIn = kRawDepth * 128, kIirOut = kIirIn + 512, kIirHand = kIirOut + 256 + 16;
+constexpr int kIirHandStride = 128 + 16;
+constexpr int kIirBytes = kIirHand + 3 * kIirHandStride;
+static_assert(kIirBytes % 128 == 64, "two blocks' accesses fill the 32 banks");
+// Blocks per CTA (one CTA per SM): 32 is one compute warp per scheduler, the
+// least latency (0.80 ms; 25 cycles a step); 64 is two, which holds half the
+// SMs for longer (1.2 ms).  The stage runs beside the demodulation, which
+// outlasts it in long captures: there the SMs it holds matter, in short ones
+// its latency does.  Whole luma and chroma decodes, 32 against 64: 144 blocks
+// 1.43 / 1.86 ms, 620 blocks 1.87 / 2.30, 793 blocks 2.37 / 2.47, 1011 blocks
+// 2.88 / 2.70, 1336 blocks 3.56 / 3.59 (from pinned host memory 3.82 / 3.70).
+// With four lanes a block and no helper warps (64 blocks a CTA, inputs read
+// by lane 0 between batches) the stage took 1.5 ms whatever the capture.
+constexpr int kBlockGroupsLow = 32;
+constexpr int kBlockGroups = 64;
+constexpr int64_t kLowLatencyBlocks = 800;
 static_assert(kChromaRowStride == kExtBatches * 32, "scratch rows hold whole chunks");
+static_assert(kChromaEdge == 27 && kIirLead == 5, "step T takes source sample T - 32");
+static_assert(kChromaExt + 2 * kIirLead == 32 * kExtBatches, "step T takes row float 32 kExtBatches - 1 - T backward");
+static_assert(32 * kIirChunks - 3 * kIirLag <= kChromaRowStride, "the last stores end inside the row");
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -105,145 +139,196 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Forward input at extended position e near the ends of the block (odd
-// extension: 2 x[0] - x[edge - e] before it, 2 x[last] - x[...] after it),
-// read from the ring (chunk q holds source samples [32 (q - 1), 32 q)).
-template <typename T>
-__device__ __noinline__ float block_edge_input(const uint8_t* ring, int e, float first, float last) {
-    if (e >= kChromaExt) return 0.0f;
-    const bool lo = e < kChromaEdge, hi = e >= kChromaEdge + kBlock;
-    const int i = lo ? kChromaEdge - e : hi ? kBlock - 2 - (e - kChromaEdge - kBlock) : e - kChromaEdge;
-    const float x = (float)reinterpret_cast<const T*>(ring + (((i >> 5) + 1) % kRingDepth) * kRingSlot)[i & 31];
-    return lo ? __fsub_rn(__fmul_rn(2.0f, first), x) : hi ? __fsub_rn(__fmul_rn(2.0f, last), x) : x;
+// int16 half `hi` of w (its sign bits flipped) as a float: 2^23 + (x + 32768)
+// as float bits, minus 2^23 + 32768 (exact)
+__device__ __forceinline__ float half_to_float(uint32_t w, bool hi) {
+    return __fadd_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, hi ? 0x7632 : 0x7610)), -8421376.0f);
 }
 
-// One pass of the block's 4-section cascade by its 4-lane group: lane s runs
-// section s on batch k - s.  kMode 0: forward over the int16 block, 1: forward
-// over the float block, 2: backward over the forward output in the row.
-// The forward pass writes sample e at row[e]; the backward pass reads row[r]
-// for sample kChromaExt - 1 - r and writes its output at row[r + kChromaRowShift]
-// (every source position is in the ring long before a later sample's output
-// lands on it).
+__device__ __forceinline__ void pair_barrier(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// Lane `s` of a block's group in a compute warp: section s over every chunk.
+// Validity of sample e = T - 5 - 32 s is checked only in the first and last
+// chunks; the products of a batch's inputs come first (they do not wait for
+// the recurrence).
+__device__ __forceinline__ void iir_compute(const float (&sec)[6], float z1, float z2, int s, uint8_t* blk, int bar) {
+    const uint8_t* in = s == 0 ? blk + kIirIn : blk + kIirHand + (s - 1) * kIirHandStride;
+    const int in_mask = s == 0 ? 511 : 127;
+    uint8_t* out = s == 3 ? blk + kIirOut : blk + kIirHand + s * kIirHandStride;
+    const int out_mask = s == 3 ? 255 : 127;
+    auto load = [&](int j, float (&x)[16]) {
+        const float4* p = reinterpret_cast<const float4*>(in + ((64 * j) & in_mask));
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float4 v = p[u];
+            x[4 * u] = v.x; x[4 * u + 1] = v.y; x[4 * u + 2] = v.z; x[4 * u + 3] = v.w;
+        }
+    };
+    // batch j of 16 steps: cur holds its inputs, nxt receives those of batch j + 1
+    auto batch = [&](bool fast, int j, float (&cur)[16], float (&nxt)[16]) {
+        load(j + 1, nxt);
+        if (fast) {
+            float p1[16], p2[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float v = cur[q];
+                cur[q] = __fmul_rn(sec[0], v);
+                p1[q] = __fmul_rn(sec[1], v);
+                p2[q] = __fmul_rn(sec[2], v);
+            }
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float f = __fadd_rn(cur[q], z1);
+                z1 = __fadd_rn(__fsub_rn(p1[q], __fmul_rn(sec[4], f)), z2);
+                z2 = __fsub_rn(p2[q], __fmul_rn(sec[5], f));
+                cur[q] = f;
+            }
+        } else {
+            const int e0 = 16 * j - kIirLead - kIirLag * s;
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+                cur[q] = e0 + q >= 0 && e0 + q < kChromaExt ? sos_step(sec, cur[q], z1, z2) : 0.0f;
+        }
+        float4* o = reinterpret_cast<float4*>(out + ((64 * j) & out_mask));
+#pragma unroll
+        for (int u = 0; u < 4; u++) o[u] = make_float4(cur[4 * u], cur[4 * u + 1], cur[4 * u + 2], cur[4 * u + 3]);
+        __syncwarp();
+    };
+    constexpr int first_fast = (kIirLead + 3 * kIirLag + 31) / 32, fast_end = (kChromaExt + kIirLead) / 32;
+    float a[16], b[16];
+    pair_barrier(bar);
+    load(0, a);
+    for (int r = 0; r < kIirChunks; r++) {
+        if (r >= first_fast && r < fast_end) {
+            batch(true, 2 * r, a, b);
+            batch(true, 2 * r + 1, b, a);
+        } else {
+            batch(false, 2 * r, a, b);
+            batch(false, 2 * r + 1, b, a);
+        }
+        pair_barrier(bar);
+    }
+}
+
+// Lane `h` (0 .. 3) of a block's group in a helper warp: an eighth of every
+// chunk is 16 bytes of int16 source, 32 bytes of floats.  kMode 0: forward
+// over the int16 block, 1: forward over the float block, 2: backward over the
+// forward output.  The forward pass writes sample e at row[5 + e]; the
+// backward pass reads its sample e there and writes it in place, at
+// row[5 + kChromaExt - 1 - e] (every source position is in the ring long
+// before an output lands on it).
 template <int kMode>
-__device__ __forceinline__ void block_pass(const float (&sec)[6], float zi0, float zi1, int s, bool active,
-                                           const void* src, float* row, uint8_t* ring, float first, float last) {
-    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
-    const float x0 = kMode == 2 ? row[kChromaExt - 1]
-                                : __fsub_rn(__fmul_rn(2.0f, first),
-                                            kMode == 0 ? (float)static_cast<const int16_t*>(src)[kChromaEdge]
-                                                       : static_cast<const float*>(src)[kChromaEdge]);
-    float z1 = __fmul_rn(zi0, x0), z2 = __fmul_rn(zi1, x0);
-    // chunk q into slot q % depth: forward q = 1 .. kBlock/32 (source [32 (q-1), 32 q)),
-    // backward q = 0 .. kExtBatches-1 (row floats [32 m, 32 m + 32), m = kExtBatches - 1 - q)
+__device__ __forceinline__ void iir_helper(int h, bool active, const void* src, float* row, uint8_t* blk, float first,
+                                           float last, int bar) {
+    const uint32_t raw_s = (uint32_t)__cvta_generic_to_shared(blk);
+    const int hr = kMode == 2 ? 3 - h : h;   // this lane's part of a source chunk
+    // source chunk q (steps [32 q, 32 q + 32)): forward q = 1 .. kBlock / 32
+    // (source [32 (q - 1), 32 q)), backward q = 0 .. kExtBatches - 1 (row
+    // floats [32 m, 32 m + 32), m = kExtBatches - 1 - q)
     auto issue = [&](int q) {
-        if (active) {
-            const uint32_t slot = ring_s + (q % kRingDepth) * kRingSlot;
+        if (active && (kMode == 2 ? q < kExtBatches : (q >= 1 && q <= kBlock / 32))) {
+            const uint32_t slot = raw_s + (q % kRawDepth) * 128;
             if (kMode == 0) {
-                if (q >= 1 && q <= kBlock / 32)
-                    cp_async16(slot + 16 * s, static_cast<const int16_t*>(src) + 32 * (q - 1) + 8 * s);
-            } else if (kMode == 1) {
-                if (q >= 1 && q <= kBlock / 32) {
-                    const float* f = static_cast<const float*>(src) + 32 * (q - 1) + 4 * s;
-                    cp_async16(slot + 16 * s, f);
-                    cp_async16(slot + 64 + 16 * s, f + 16);
-                }
-            } else if (q >= 0 && q < kExtBatches) {
-                const float* f = row + 32 * (kExtBatches - 1 - q) + 4 * s;
-                cp_async16(slot + 16 * s, f);
-                cp_async16(slot + 64 + 16 * s, f + 16);
+                cp_async16(slot + 16 * hr, static_cast<const int16_t*>(src) + 32 * (q - 1) + 8 * hr);
+            } else {
+                const float* g = (kMode == 1 ? static_cast<const float*>(src) + 32 * (q - 1)
+                                             : row + 32 * (kExtBatches - 1 - q)) + 8 * hr;
+                cp_async16(slot + 32 * hr, g);
+                cp_async16(slot + 32 * hr + 16, g + 4);
             }
         }
         cp_async_commit();
     };
+    auto raw = [&](int i) -> float {   // source sample i of the block
+        const uint8_t* slot = blk + (((i >> 5) + 1) % kRawDepth) * 128;
+        return kMode == 0 ? (float)reinterpret_cast<const int16_t*>(slot)[i & 31]
+                          : reinterpret_cast<const float*>(slot)[i & 31];
+    };
+    // steps [32 q + 8 h, + 8) of the input ring
+    auto prepare = [&](int q) {
+        float4* o = reinterpret_cast<float4*>(blk + kIirIn + (q & 3) * 128 + 32 * h);
+        const uint8_t* slot = blk + (q % kRawDepth) * 128;
+        if (kMode != 2 && (q < 1 || q > kBlock / 32)) {
+            // odd extension: 2 x[0] - x[edge - e] before the block, 2 x[last] - x[...] after it
+            float v[8];
 #pragma unroll
-    for (int q = 0; q < kRingDepth - 1; q++) issue(q);
-    float a[32], b[32];
-#pragma unroll
-    for (int q = 0; q < 32; q++) a[q] = b[q] = 0.0f;
-    // batch k: chunks k and k + 1 are complete (the ones after them in flight)
-    auto batch = [&](int k, float (&cur)[32], float (&nxt)[32]) {
-        cp_async_wait<kRingDepth - 3>();
-        __syncwarp();
-        issue(k + kRingDepth - 1);   // into the slot of chunk k - 1, read last batch
-        if (s == 0 && k < kExtBatches) {
-            const uint8_t* r0 = ring + (k % kRingDepth) * kRingSlot;
-            const uint8_t* r1 = ring + ((k + 1) % kRingDepth) * kRingSlot;
-            if (kMode == 2) {
-                constexpr int top = (kChromaExt - 1) % 32;
-                const float* f0 = reinterpret_cast<const float*>(r0);
-                const float* f1 = reinterpret_cast<const float*>(r1);
-#pragma unroll
-                for (int q = 0; q < 32; q++) cur[q] = q <= top ? f0[top - q] : f1[top + 32 - q];
-            } else if (k >= 1 && k < kBlock / 32) {
-                constexpr int lead = 32 - kChromaEdge;
-                if (kMode == 0) {
-                    const int16_t* h0 = reinterpret_cast<const int16_t*>(r0);
-                    const int16_t* h1 = reinterpret_cast<const int16_t*>(r1);
-#pragma unroll
-                    for (int q = 0; q < 32; q++) cur[q] = (float)(q < kChromaEdge ? h0[q + lead] : h1[q - kChromaEdge]);
-                } else {
-                    const float* f0 = reinterpret_cast<const float*>(r0);
-                    const float* f1 = reinterpret_cast<const float*>(r1);
-#pragma unroll
-                    for (int q = 0; q < 32; q++) cur[q] = q < kChromaEdge ? f0[q + lead] : f1[q - kChromaEdge];
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < 32; q++)
-                    cur[q] = kMode == 0 ? block_edge_input<int16_t>(ring, 32 * k + q, first, last)
-                                        : block_edge_input<float>(ring, 32 * k + q, first, last);
+            for (int u = 0; u < 8; u++) {
+                const int e = 32 * q + 8 * h + u - kIirLead;
+                v[u] = e < 0 || e >= kChromaExt ? 0.0f
+                       : e < kChromaEdge        ? __fsub_rn(__fmul_rn(2.0f, first), raw(kChromaEdge - e))
+                                                : __fsub_rn(__fmul_rn(2.0f, last),
+                                                            raw(kBlock - 2 - (e - kChromaEdge - kBlock)));
             }
-        }
-        const int i0 = 32 * (k - s);
-        if (i0 >= 0 && i0 + 32 <= kChromaExt) {
-#pragma unroll
-            for (int q = 0; q < 32; q++) {
-                cur[q] = sos_step(sec, cur[q], z1, z2);
-                nxt[q] = __shfl_up_sync(kFull, cur[q], 1, 4);
-            }
+            o[0] = make_float4(v[0], v[1], v[2], v[3]);
+            o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else if (kMode == 0) {
+            const uint4 x = *reinterpret_cast<const uint4*>(slot + 16 * hr);
+            const uint32_t w[4] = {x.x ^ 0x80008000u, x.y ^ 0x80008000u, x.z ^ 0x80008000u, x.w ^ 0x80008000u};
+            o[0] = make_float4(half_to_float(w[0], false), half_to_float(w[0], true), half_to_float(w[1], false),
+                               half_to_float(w[1], true));
+            o[1] = make_float4(half_to_float(w[2], false), half_to_float(w[2], true), half_to_float(w[3], false),
+                               half_to_float(w[3], true));
         } else {
-#pragma unroll
-            for (int q = 0; q < 32; q++) {
-                const int i = i0 + q;
-                cur[q] = (i >= 0 && i < kChromaExt) ? sos_step(sec, cur[q], z1, z2) : 0.0f;
-                nxt[q] = __shfl_up_sync(kFull, cur[q], 1, 4);
-            }
-        }
-        const int kk = k - 3;   // the last section's batch
-        if (s == 3 && active && kk >= 0 && kk < kExtBatches) {
-            if (kMode != 2) {
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    *reinterpret_cast<float4*>(row + 32 * kk + 4 * u) =
-                        make_float4(cur[4 * u], cur[4 * u + 1], cur[4 * u + 2], cur[4 * u + 3]);
-            } else {
-                const int base = kChromaExt + kChromaRowShift - 32 - 32 * kk;   // a multiple of 4
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (base + 4 * u >= 0)
-                        *reinterpret_cast<float4*>(row + base + 4 * u) =
-                            make_float4(cur[31 - 4 * u], cur[30 - 4 * u], cur[29 - 4 * u], cur[28 - 4 * u]);
-            }
+            const float4* x = reinterpret_cast<const float4*>(slot + 32 * hr);
+            const float4 u = x[0], v = x[1];
+            o[0] = kMode == 1 ? u : make_float4(v.w, v.z, v.y, v.x);
+            o[1] = kMode == 1 ? v : make_float4(u.w, u.z, u.y, u.x);
         }
     };
-    constexpr int nb = kExtBatches + 3;
-    for (int k = 0; k < nb; k += 2) {
-        batch(k, a, b);
-        batch(k + 1, b, a);
+    // lane 3's outputs of chunk r: row floats [32 (r - 3), + 32) forward,
+    // [32 (kIirChunks - 1 - r), + 32) backward
+    auto store = [&](int r) {
+        if (!active || r < 3) return;
+        const float4* y = reinterpret_cast<const float4*>(blk + kIirOut + (r & 1) * 128 + 32 * h);
+        const float4 u = y[0], v = y[1];
+        float4* o = reinterpret_cast<float4*>(row + 32 * (kMode == 2 ? kIirChunks - 1 - r : r - 3) + 8 * hr);
+        o[0] = kMode != 2 ? u : make_float4(v.w, v.z, v.y, v.x);
+        o[1] = kMode != 2 ? v : make_float4(u.w, u.z, u.y, u.x);
+    };
+#pragma unroll 1
+    for (int q = 0; q < kRawDepth - 1; q++) issue(q);
+    cp_async_wait<kRawDepth - 3>();   // chunks 0 and 1
+    __syncwarp();
+    prepare(0);
+    prepare(1);
+    pair_barrier(bar);
+    // while the compute warp runs chunk r: chunk r + 2 into the input ring, the
+    // outputs of chunk r - 1, and the source of chunk r + 15 into the slot of
+    // chunk r - 1
+    for (int r = 0; r < kIirChunks; r++) {
+        issue(r + kRawDepth - 1);
+        cp_async_wait<kRawDepth - 3>();   // chunk r + 2
+        if (kMode != 2 && r + 2 > kBlock / 32) __syncwarp();   // the extension reads the whole chunk
+        prepare(r + 2);
+        store(r - 1);
+        pair_barrier(bar);
     }
+    store(kIirChunks - 1);
     cp_async_wait_all();
 }
 
-// One 4-lane group per RF block: the forward pass over the odd extension of
-// the block into its scratch row, then the backward pass in place.
-__global__ void __launch_bounds__(4 * kBlockGroups) k_chroma_block_iir(ChromaBlockParams p) {
-    extern __shared__ __align__(128) uint8_t rings[];   // [kBlockGroups * kRingBytes]
-    const int s = threadIdx.x & 3, g = threadIdx.x >> 2;
-    const int64_t j = (int64_t)blockIdx.x * kBlockGroups + g;
+// Forward over the odd extension of each block into its scratch row, then
+// backward in place.  The first half of the warps computes, the second helps.
+__global__ void __launch_bounds__(8 * kBlockGroups) k_chroma_block_iir(ChromaBlockParams p) {
+    extern __shared__ __align__(128) uint8_t iir_smem[];   // [blocks of the CTA * kIirBytes]
+    const int half = blockDim.x >> 1, t = threadIdx.x < half ? threadIdx.x : threadIdx.x - half;
+    const bool helper = threadIdx.x >= half;
+    const int s = t & 3, g = t >> 2, bar = 1 + (t >> 5);
+    const int64_t j = (int64_t)blockIdx.x * (half >> 2) + g;
     const bool active = j < p.nblocks;
     const int64_t base = (p.first_block + (active ? j : 0)) * kStride;
     float* row = p.scratch + (active ? j : 0) * kChromaRowStride;
-    uint8_t* ring = rings + g * kRingBytes;
+    uint8_t* blk = iir_smem + g * kIirBytes;
+    const float first = p.rf32 ? p.rf32[base] : (float)p.rf16[base];
+    if (helper) {
+        const float last = p.rf32 ? p.rf32[base + kBlock - 1] : (float)p.rf16[base + kBlock - 1];
+        if (p.rf32) iir_helper<1>(s, active, p.rf32 + base, row, blk, first, last, bar);
+        else iir_helper<0>(s, active, p.rf16 + base, row, blk, first, last, bar);
+        __threadfence();   // the forward outputs before the backward pass's copies of them
+        __syncthreads();
+        iir_helper<2>(s, active, nullptr, row, blk, 0.0f, 0.0f, bar);
+        return;
+    }
     // section s of the cascade (selected with constant indices: a dynamic
     // index into the parameter block would copy it to local memory)
     float sec[6];
@@ -252,48 +337,46 @@ __global__ void __launch_bounds__(4 * kBlockGroups) k_chroma_block_iir(ChromaBlo
         sec[k] = s == 0 ? p.c.sec[0][k] : s == 1 ? p.c.sec[1][k] : s == 2 ? p.c.sec[2][k] : p.c.sec[3][k];
     const float zi0 = s == 0 ? p.c.zi[0][0] : s == 1 ? p.c.zi[1][0] : s == 2 ? p.c.zi[2][0] : p.c.zi[3][0];
     const float zi1 = s == 0 ? p.c.zi[0][1] : s == 1 ? p.c.zi[1][1] : s == 2 ? p.c.zi[2][1] : p.c.zi[3][1];
-    if (p.rf32) {
-        const float* x = p.rf32 + base;
-        block_pass<1>(sec, zi0, zi1, s, active, x, row, ring, x[0], x[kBlock - 1]);
-    } else {
-        const int16_t* x = p.rf16 + base;
-        block_pass<0>(sec, zi0, zi1, s, active, x, row, ring, (float)x[0], (float)x[kBlock - 1]);
+    // the steady state for the pass's first sample
+    float x0 = __fsub_rn(__fmul_rn(2.0f, first), p.rf32 ? p.rf32[base + kChromaEdge] : (float)p.rf16[base + kChromaEdge]);
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        iir_compute(sec, __fmul_rn(zi0, x0), __fmul_rn(zi1, x0), s, blk, bar);
+        if (pass == 0) {
+            __syncthreads();
+            x0 = __ldcg(row + kIirLead + kChromaExt - 1);
+        }
     }
-    // the forward outputs of lane 3 before the other lanes' copies of them
-    __threadfence();
-    __syncwarp();
-    block_pass<2>(sec, zi0, zi1, s, active, nullptr, row, ring, 0.0f, 0.0f);
 }
 
 // One warp per block: the float mean of the rolled block in the reference's
-// 32-accumulator order (lane a sums rolled samples a, a + 32, ... in order),
-// then the stitched span minus the mean.
-__global__ void __launch_bounds__(32) k_chroma_block_dc(ChromaBlockParams p) {
+// 32-accumulator order (lane a sums rolled samples a, a + 32, ... in order).
+__global__ void __launch_bounds__(32) k_chroma_block_mean(ChromaBlockParams p) {
     const int64_t j = blockIdx.x;
     const int lane = threadIdx.x;
     const float* y = p.scratch + j * (int64_t)kChromaRowStride + kChromaEdge + kChromaRowShift;
     const int move = p.move;
     float acc = 0.0f;
-    for (int i0 = 0; i0 < kBlock; i0 += 32 * 16) {
-        float v[16];
+    for (int i0 = 0; i0 < kBlock; i0 += 32 * 32) {
+        float v[32];
 #pragma unroll
-        for (int q = 0; q < 16; q++) v[q] = y[(i0 + q * 32 + lane - move) & (kBlock - 1)];
+        for (int q = 0; q < 32; q++) v[q] = y[(i0 + q * 32 + lane - move) & (kBlock - 1)];
 #pragma unroll
-        for (int q = 0; q < 16; q++) acc = __fadd_rn(acc, v[q]);
+        for (int q = 0; q < 32; q++) acc = __fadd_rn(acc, v[q]);
     }
     // lanes[l] = (acc[l] + acc[8 + l]) + (acc[16 + l] + acc[24 + l]), then a tree over 8 lanes
     float t = __fadd_rn(acc, __shfl_down_sync(kFull, acc, 8));
     float l8 = __fadd_rn(t, __shfl_down_sync(kFull, t, 16));
     for (int c = 8; c > 1; c /= 2) l8 = __fadd_rn(l8, __shfl_down_sync(kFull, l8, c / 2));
-    const float mean = __fdiv_rn(__shfl_sync(kFull, l8, 0), (float)kBlock);
-    float* out = p.out + (p.first_block + j) * kStride;
-    for (int i0 = 0; i0 < kStride; i0 += 32 * 8) {
-        float v[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = y[(kCut + i0 + q * 32 + lane - move) & (kBlock - 1)];
-#pragma unroll
-        for (int q = 0; q < 8; q++) out[i0 + q * 32 + lane] = __fsub_rn(v[q], mean);
-    }
+    if (lane == 0) p.mean[j] = __fdiv_rn(l8, (float)kBlock);
+}
+
+// The stitched channel: the kept samples of the rolled blocks minus the means.
+__global__ void __launch_bounds__(256) k_chroma_block_stitch(ChromaBlockParams p, float* out) {
+    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, j = at / kStride;
+    const int s = (int)(at - j * kStride);
+    const float* y = p.scratch + j * (int64_t)kChromaRowStride + chroma_row_offset(p.move);
+    out[at] = __fsub_rn(y[s], p.mean[j]);
 }
 
 // ---------------------------------------------------------------- burst probes
@@ -940,14 +1023,20 @@ __global__ void __launch_bounds__(320) k_chroma_gain(ChromaFieldParams p) {
 
 }  // namespace
 
-int chroma_block_ctas(int64_t nblocks) { return (int)((nblocks + kBlockGroups - 1) / kBlockGroups); }
+static int block_groups(int64_t nblocks) {
+    return nblocks <= kLowLatencyBlocks ? kBlockGroupsLow : kBlockGroups;
+}
+int chroma_block_ctas(int64_t nblocks) {
+    const int g = block_groups(nblocks);
+    return (int)((nblocks + g - 1) / g);
+}
 
 cudaError_t prepare_chroma_kernels() {
     // the block stage's rings above the default 48 KB of shared memory; all of
     // the SM's shared memory for the probe rows, so a decode's probe warps fit
     // in one wave
     cudaError_t e = cudaFuncSetAttribute(k_chroma_block_iir, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kBlockGroups * kRingBytes);
+                                         kBlockGroups * kIirBytes);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_chroma_probe, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
 }
@@ -958,9 +1047,21 @@ cudaError_t launch_chroma_blocks(const ChromaBlockParams& p, cudaStream_t s) {
         (reinterpret_cast<uintptr_t>(p.rf32 ? (const void*)p.rf32 : (const void*)p.rf16) & 15u) != 0 ||
         (reinterpret_cast<uintptr_t>(p.scratch) & 15u) != 0)
         return cudaErrorInvalidValue;
-    constexpr int smem = kBlockGroups * kRingBytes;   // opted in by prepare_chroma_kernels
-    k_chroma_block_iir<<<(unsigned)((p.nblocks + kBlockGroups - 1) / kBlockGroups), 4 * kBlockGroups, smem, s>>>(p);
-    k_chroma_block_dc<<<(unsigned)p.nblocks, 32, 0, s>>>(p);
+    const int groups = block_groups(p.nblocks);   // shared memory opted in by prepare_chroma_kernels
+    k_chroma_block_iir<<<(unsigned)chroma_block_ctas(p.nblocks), 8 * groups, groups * kIirBytes, s>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_chroma_means(const ChromaBlockParams& p, cudaStream_t s) {
+    if (p.nblocks <= 0) return cudaSuccess;
+    k_chroma_block_mean<<<(unsigned)p.nblocks, 32, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_chroma_stitch(const ChromaBlockParams& p, float* out, cudaStream_t s) {
+    if (p.nblocks <= 0) return cudaSuccess;
+    static_assert(kStride % 256 == 0, "whole CTAs");
+    k_chroma_block_stitch<<<(unsigned)(p.nblocks * (kStride / 256)), 256, 0, s>>>(p, out);
     return cudaGetLastError();
 }
 

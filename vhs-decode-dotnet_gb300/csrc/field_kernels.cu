@@ -1281,6 +1281,7 @@ __global__ void k_tbc_consts(TbcParams p) {
 
 constexpr int kTbcFastMaxThreads = 320;
 constexpr int kTbcStageBytes = 96 * 1024;   // most shared memory for a line's source
+static_assert(kTbcStageBytes / (int)sizeof(float) < kStride, "a staged stretch meets one block end at most");
 constexpr int kTapRow = 16;   // floats of a sample's weight row
 // Where four taps 4 c .. 4 c + 3 of the warp's sample i lie in its row: both
 // the quads' stores and the lanes' loads of a row fill all 32 banks.
@@ -1411,11 +1412,24 @@ __device__ __forceinline__ void tap_sums(const float (&x)[16], const float (&y)[
 //   sample and 32 bytes a lane, so a row pair is one 128-byte access; the quad
 //   interpolates and leaves the 16 weights in the sample's shared row;
 // * each lane then sums its own sample alone, luma (and with kPair the chroma,
-//   src2 -> out2_f32, with the same weights) in packed pair additions.
+//   -> out2_f32, with the same weights) in packed pair additions.
+// The chroma is read from the block stage's rows (kRows: instead of the
+// stream): stitched, rolled and its mean taken off as it is staged.
 // Split over a quad, with a shuffled tree of pair additions per sample and
 // 4-byte source loads, the same sums cost 1000 instructions a luma and chroma
 // sample pair.
-template <bool kPair>
+struct RowSource {
+    const float* row;     // the span's first row
+    const float* mean;
+    int offset;
+    // sample idx >= 0 of the span (spans start on a block)
+    __device__ __forceinline__ float at(int idx) const {
+        const int b = idx / kStride;
+        return __fsub_rn(__ldg(row + (int64_t)b * (kChromaRowStride - kStride) + offset + idx), __ldg(mean + b));
+    }
+};
+
+template <bool kPair, bool kRows>
 __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float* stream, int64_t stream_len,
                                                                     TbcParams p, int stage_cap) {
     extern __shared__ __align__(16) float tbc_smem[];
@@ -1430,7 +1444,11 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
     const TbcLineConsts& c = *reinterpret_cast<const TbcLineConsts*>(
         p.line_consts + ((int64_t)f * p.out_lines + ol) * kTbcLineConstsBytes);
     uint16_t* out = p.out_u16 ? p.out_u16 + ((int64_t)f * p.out_lines + ol) * p.outlen : nullptr;
-    const float* src2 = p.src2 ? p.src2 + s0 : nullptr;
+    RowSource chroma{};
+    if (kPair || kRows) {
+        const int64_t b0 = s0 / kStride;
+        chroma = RowSource{p.rows + b0 * kChromaRowStride, p.row_mean + b0, p.row_offset};
+    }
     float* out2 = p.out2_f32 ? p.out2_f32 + ((int64_t)f * p.out_lines + ol) * p.outlen : nullptr;
     float* outf32 = p.out_f32 ? p.out_f32 + ((int64_t)f * p.out_lines + ol) * p.out_stride - p.x0 : nullptr;
     const int kx1 = p.x1 > 0 ? p.x1 : p.outlen;
@@ -1444,12 +1462,33 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
     const int first = tap_pos(c, p.x0).ci - 7, last = tap_pos(c, kx1 - 1).ci - 7;
     const int lo = min(first, last) & ~3;
     const int len = ((max(first, last) + 19 - lo) + 3) & ~3;
-    const bool staged = min(first, last) >= 0 && len > 0 && len <= stage_cap && lo + len <= n32;
+    const int lo2 = lo - ((lo + chroma.offset) & 3);   // the same for the chroma, on its rows' alignment
+    const bool staged = min(first, last) >= 0 && len > 0 && len + 4 <= stage_cap && lo + len <= n32;
     if (staged) {
-        for (int i = 4 * threadIdx.x; i < len; i += 4 * blockDim.x) {
-            *reinterpret_cast<float4*>(stage + i) = __ldg(reinterpret_cast<const float4*>(src + lo + i));
-            if (kPair)
-                *reinterpret_cast<float4*>(stage + stage_cap + i) = __ldg(reinterpret_cast<const float4*>(src2 + lo + i));
+        if (!kRows)
+            for (int i = 4 * threadIdx.x; i < len; i += 4 * blockDim.x)
+                *reinterpret_cast<float4*>(stage + i) = __ldg(reinterpret_cast<const float4*>(src + lo + i));
+        if (kPair || kRows) {
+            // four floats at a time on the rows' alignment, from lo2 on; a
+            // stretch meets one block end at most (stage_cap < kStride)
+            float* to = stage + (kPair ? stage_cap : 0);
+            const int b0 = lo / kStride, end0 = (b0 + 1) * kStride - lo2;
+            const float* r0 = chroma.row + (int64_t)b0 * (kChromaRowStride - kStride) + chroma.offset + lo2;
+            const float* r1 = r0 + (kChromaRowStride - kStride);
+            static_assert((kChromaRowStride - kStride) % 4 == 0, "rows keep the alignment");
+            const float m0 = __ldg(chroma.mean + b0), m1 = end0 < len + 4 ? __ldg(chroma.mean + b0 + 1) : 0.0f;
+            for (int i = 4 * threadIdx.x; i < len + 4; i += 4 * blockDim.x) {
+                float4 v = __ldg(reinterpret_cast<const float4*>((i < end0 ? r0 : r1) + i));
+                if (i < end0 && i + 4 > end0) {   // the block ends inside
+                    const float4 w = __ldg(reinterpret_cast<const float4*>(r1 + i));
+                    if (i + 1 >= end0) v.y = w.y;
+                    if (i + 2 >= end0) v.z = w.z;
+                    v.w = w.w;
+                }
+                *reinterpret_cast<float4*>(to + i) =
+                    make_float4(__fsub_rn(v.x, i < end0 ? m0 : m1), __fsub_rn(v.y, i + 1 < end0 ? m0 : m1),
+                                __fsub_rn(v.z, i + 2 < end0 ? m0 : m1), __fsub_rn(v.w, i + 3 < end0 ? m0 : m1));
+            }
         }
         __syncthreads();
     }
@@ -1475,8 +1514,8 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
         float x[16], x2[16];
         const int start = tp.ci - 7;
         if (staged) {
-            load_taps(stage + (start - lo), x);
-            if (kPair) load_taps(stage + stage_cap + (start - lo), x2);
+            load_taps(stage + (start - (kRows ? lo2 : lo)), x);
+            if (kPair) load_taps(stage + stage_cap + (start - lo2), x2);
         } else {
 #pragma unroll
             for (int t = 0; t < 16; t++) {
@@ -1486,8 +1525,8 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
                     if (idx < 0) idx += n32;
                     idx = idx < 0 ? 0 : (idx > n32 - 1 ? n32 - 1 : idx);
                 }
-                x[t] = __ldg(src + idx);
-                if (kPair) x2[t] = __ldg(src2 + idx);
+                x[t] = kRows ? chroma.at(idx) : __ldg(src + idx);
+                if (kPair) x2[t] = chroma.at(idx);
             }
         }
         __syncwarp();
@@ -1535,9 +1574,12 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
 
 cudaError_t prepare_tbc_kernels() {
     const int most = kTbcStageBytes + kTbcFastMaxThreads * kTapRow * (int)sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_tbc_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_tbc_fast<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    cudaError_t e = cudaFuncSetAttribute(k_tbc_fast<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_tbc_fast<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_tbc_fast<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e;
 }
 
 // pw must hold (1-alpha)^(k+1) for k in [0, outlen) when smoothing > 0.
@@ -1562,14 +1604,15 @@ cudaError_t launch_tbc_pw(const T* stream, int64_t stream_len, const TbcParams& 
         const int passes = (width + kTbcFastMaxThreads - 1) / kTbcFastMaxThreads;
         const int threads = ((width + passes - 1) / passes + 31) / 32 * 32;
         // the stage holds the window's stretch of a line 4 % longer than nominal
-        const int fit = ((int)(p.nominal * 1.04 * width / p.outlen) + 48) & ~3;
-        const int room = (kTbcStageBytes / (p.src2 ? 2 : 1) / (int)sizeof(float)) & ~3;
+        const int fit = ((int)(p.nominal * 1.04 * width / p.outlen) + 52) & ~3;
+        const bool pair = p.rows && p.out2_f32;
+        const int room = (kTbcStageBytes / (pair ? 2 : 1) / (int)sizeof(float)) & ~3;
         const int cap = fit < room ? fit : room;
-        const size_t smem = ((size_t)threads * kTapRow + (size_t)cap * (p.src2 ? 2 : 1)) * sizeof(float);
-        if (p.src2)
-            k_tbc_fast<true><<<grid, threads, smem, s>>>(reinterpret_cast<const float*>(stream), stream_len, p, cap);
-        else
-            k_tbc_fast<false><<<grid, threads, smem, s>>>(reinterpret_cast<const float*>(stream), stream_len, p, cap);
+        const size_t smem = ((size_t)threads * kTapRow + (size_t)cap * (pair ? 2 : 1)) * sizeof(float);
+        const float* src = reinterpret_cast<const float*>(stream);
+        if (pair) k_tbc_fast<true, false><<<grid, threads, smem, s>>>(src, stream_len, p, cap);
+        else if (p.rows) k_tbc_fast<false, true><<<grid, threads, smem, s>>>(src, stream_len, p, cap);
+        else k_tbc_fast<false, false><<<grid, threads, smem, s>>>(src, stream_len, p, cap);
     } else {
         k_tbc<T><<<grid, 256, 0, s>>>(stream, stream_len, p, pw);
     }

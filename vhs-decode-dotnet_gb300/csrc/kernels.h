@@ -189,9 +189,14 @@ struct TbcParams {
     float* out_f32;             // optional float output [nfields * out_lines * out_stride]:
                                 // samples x0 .. x1-1 of each line at (k - x0)
     int x0, x1, out_stride;     // line window of out_f32 (x1 = 0: the whole line)
-    const float* src2;          // optional second float stream rendered with the same
-    float* out2_f32;            //   positions and weights (the chroma beside the luma),
-                                //   [nfields * out_lines * outlen] (fast float kernel only)
+    // optional chroma channel in rows (ChromaBlockParams; fast float kernel
+    // only), row_offset its chroma_row_offset: the source instead of the
+    // stream, or with out2_f32 a second one rendered beside it with the same
+    // positions and weights to out2_f32 [nfields * out_lines * outlen]
+    const float* rows;
+    const float* row_mean;
+    int row_offset;
+    float* out2_f32;
     double* level_work;         // [nfields * (max_first_line + out_lines)] line factors
     unsigned char* line_consts; // [nfields * out_lines * kTbcLineConstsBytes] float-pair line plans
                                 // of the fast float kernel (null: binary64 kernel)
@@ -218,18 +223,23 @@ struct ChromaCascade {
 
 // The odd extension of an RF block before its chroma band-pass: the default
 // pad length of a 4-section filter with no zero end coefficients,
-// 3 * (2 * 4 + 1).  Scratch rows of the block stage hold the extended block
-// in whole 32-float chunks, the backward pass's output starting kChromaRowShift
-// floats in (so its vector stores are 16-byte aligned).
+// 3 * (2 * 4 + 1).  Rows of the block stage hold the extended block in whole
+// 32-float chunks, starting kChromaRowShift floats in (so the vector accesses
+// of both passes are 16-byte aligned).
 constexpr int kChromaEdge = 27;
 constexpr int kChromaExt = kBlock + 2 * kChromaEdge;
 constexpr int kChromaRowStride = (kChromaExt + 31) / 32 * 32;
-constexpr int kChromaRowShift = (4 - kChromaExt % 4) % 4;
+constexpr int kChromaRowShift = 5;
+// The row float of the first kept sample of a block rolled by `move`
+// (|move| <= kCut: the kept samples do not wrap).
+__host__ __device__ inline int chroma_row_offset(int move) { return kChromaRowShift + kChromaEdge + kCut - move; }
 
 // Chroma channel of blocks [first_block, first_block + nblocks): the RF block
-// band-passed, rolled by `move` and its float mean removed, stitched like the
-// demodulated channels (stream index b*30720 + n - 1024).  The capture pointer
-// is 16-byte aligned.
+// band-passed into its row, the float mean of the block rolled by `move`
+// beside it; sample s < kStride of block j of the stitched channel (stream
+// index b*30720 + n - 1024, like the demodulated channels) is
+// row j [chroma_row_offset(move) + s] - mean[j].  The capture pointer is
+// 16-byte aligned.
 struct ChromaBlockParams {
     const int16_t* rf16;       // capture at the decode rate (int16), or
     const float* rf32;         //   float (read when set)
@@ -237,14 +247,18 @@ struct ChromaBlockParams {
     ChromaCascade c;
     int move;
     float* scratch;            // [nblocks * kChromaRowStride]
-    float* out;                // stitched chroma stream
+    float* mean;               // [nblocks]
 };
-constexpr int kChromaBlockKernels = 2;
+constexpr int kChromaBlockKernels = 2;   // band-pass, means
 // Kernel attributes of the chroma kernels (once per device, outside any capture).
 cudaError_t prepare_chroma_kernels();
 // CTAs (one per SM) of the chroma block stage for nblocks blocks.
 int chroma_block_ctas(int64_t nblocks);
+// The band-pass into the rows; the means of the complete rows; the stitched
+// channel.
 cudaError_t launch_chroma_blocks(const ChromaBlockParams& p, cudaStream_t stream);
+cudaError_t launch_chroma_means(const ChromaBlockParams& p, cudaStream_t stream);
+cudaError_t launch_chroma_stitch(const ChromaBlockParams& p, float* out, cudaStream_t stream);
 
 // Per-field chroma stages of a field batch (every array offset to the batch).
 struct ChromaFieldParams {

@@ -232,7 +232,9 @@ struct vhsdecode_gb300_session {
     bool chroma_alloc = false;
     bool want_chroma = false;            // the current decode renders chroma
     vhsd::ChromaDesign cd;
-    DevBuf<float> c32;                   // stitched chroma stream
+    DevBuf<float> c32;                   // stitched chroma stream (made by copy_stream)
+    bool c32_valid = false;              //   it holds the last decode's channel
+    DevBuf<float> c_mean;                // means of the chroma blocks
     DevBuf<float> c_scratch;             // block band-pass passes [max_blocks * (kBlock + 2 edge)]
     DevBuf<float> c_het, c_bsin, c_bcos; // field tables
     DevBuf<float> c_ana;                 // line-1 chroma TBC, probe windows
@@ -249,7 +251,8 @@ struct vhsdecode_gb300_session {
     // the chroma block band-pass runs on its own stream beside the demod
     cudaStream_t chroma_stream = nullptr;
     cudaEvent_t chroma_go = nullptr, chroma_done = nullptr;
-    bool chroma_pending = false;         // chroma blocks queued for this decode
+    int64_t chroma_blocks = 0;           // blocks band-passed for the last decode ...
+    bool chroma_means = false;           //   and their means queued
     // host results
     std::vector<FieldRec> fields;
     int64_t last_blocks = 0;
