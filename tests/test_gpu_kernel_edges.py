@@ -66,3 +66,33 @@ def test_chroma_block_stage_edges(gpu, nblocks, dtype):
         for b in sorted({0, min(nblocks - 1, 31), min(nblocks - 1, 32), min(nblocks - 1, 64), nblocks - 1}):
             want = chroma.chroma_stream(rf, cp, b, 1)
             assert np.array_equal(s.stream(3, b * STRIDE, STRIDE), want), b
+
+
+@pytest.mark.parametrize("tape,nblocks", [("VHS", 1), ("VHS", 128), ("VHS", 129), ("SVHS", 129)])
+def test_fp64_batches(gpu, tape, nblocks):
+    # the double-precision demodulator takes the blocks in batches (at most 128
+    # of equal size): a block's samples are the same wherever it lies in a
+    # batch, and within 1 Hz of the oracle's (the bound of the stream tests;
+    # both compute in binary64, whose rounding is below 1e-6 Hz, but a float
+    # angle beside a rounding boundary moves a sample by up to 0.4 Hz).  Dropouts
+    # make some blocks take the spike repair.
+    from oracle import demod, filters, formats
+    from vhsd_gb300 import native, synth
+    make = synth.pal_svhs if tape == "SVHS" else synth.pal_vhs
+    rf, _ = synth.generate(make(fields=4, seed=8, snr_db=40.0, dropouts=40))
+    rf = np.resize(rf, (nblocks - 1) * STRIDE + BLOCK)
+    fmt = formats.get("PAL", tape)
+    filt = filters.FilterSet(fmt, 40e6)
+    dmax = (fmt["sys"]["ire0"] + fmt["sys"]["hz_ire"] * 100.0) * 2.0
+    kw = dict(precision=native.PRECISION_FP64_PLAIN,
+              tape_format=native.FORMAT_SVHS if tape == "SVHS" else native.FORMAT_VHS)
+    with native.Session(native.PROFILE_PAL, len(rf), **kw) as s:
+        s.decode(rf, demod_only=True)
+        for b in sorted({0, nblocks // 2 - 1, nblocks // 2, nblocks - 1} - {-1}):
+            got = [s.stream(c, b * STRIDE, STRIDE) for c in range(3)]
+            with native.Session(native.PROFILE_PAL, BLOCK, **kw) as one:
+                one.decode(rf[b * STRIDE:b * STRIDE + BLOCK], demod_only=True)
+                for c in range(3):
+                    assert np.array_equal(got[c], one.stream(c, 0, STRIDE)), (b, c)
+            want = demod.demod_stream(rf, filt, 40e6, dmax, b, 1)
+            assert np.max(np.abs(got[0] - want[0])) < 1.0 and np.max(np.abs(got[1] - want[1])) < 1.0, b

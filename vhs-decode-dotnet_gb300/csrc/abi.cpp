@@ -256,13 +256,16 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
             s->sub64.alloc(H);
             ck(cudaMemcpy(s->sub64.p, hv.data(), H * sizeof(double2), cudaMemcpyHostToDevice), "upload");
         }
-        s->pwork.alloc(4 * (size_t)kBlock);
-        s->pdwork.alloc(3 * (size_t)kBlock);
-        s->pfwork.alloc(kBlock + 16);
-        s->pflag.alloc(4);
-        s->pmask.alloc(1024);
-        s->pblk.alloc(1);
-        ck(cudaMemset(s->pflag.p, 0, 4 * sizeof(int)), "memset");
+        const size_t batch = (size_t)std::min<int64_t>(std::max<int64_t>(1, s->max_blocks), kPlainBatch);
+        s->pwork.alloc(3 * batch * kBlock);
+        s->pdwork.alloc(3 * batch * kBlock);
+        s->pfwork.alloc(batch * kBlock);
+        s->pflag.alloc(batch);
+        s->pmask.alloc(batch * (kBlock / 32));
+        s->ptwiddle.alloc(kBlock);
+        ck(cudaMemset(s->pflag.p, 0, batch * sizeof(int)), "memset");
+        ck(make_fp64_twiddles(s->ptwiddle.p, s->own_stream), "twiddles");
+        ck(cudaStreamSynchronize(s->own_stream), "sync");
     }
     int64_t pslots = pulse_count_slots(stream_cap);
     s->pc_counts.alloc(pslots);
@@ -502,7 +505,6 @@ void session_free(vhsdecode_gb300_session* s) {
         if (e) cudaEventDestroy(e);
     if (s->chroma_stream) cudaStreamDestroy(s->chroma_stream);
     if (s->demod_cycles) cudaFree(s->demod_cycles);
-    if (s->plain_graph) cudaGraphExecDestroy(s->plain_graph);
     for (auto& ev : s->ev) if (ev) cudaEventDestroy(ev);
     for (auto* v : {&s->seg_done, &s->seg_copied, &s->seg_pulsed, &s->seg_dem, &s->seg_demod_end})
         for (auto& ev : *v) if (ev) cudaEventDestroy(ev);
@@ -702,32 +704,19 @@ void run_demod(vhsdecode_gb300_session* s, const int16_t* rf_dev, int64_t nblock
         p.fwork = s->pfwork.p;
         p.flag = s->pflag.p;
         p.mask = s->pmask.p;
-        p.blk = s->pblk.p;
+        p.twiddle = s->ptwiddle.p;
         if (s->sub64.p) {
             p.sub = sub_params<double, double2>(s->fmt, s->filt);
             p.sub.high = s->sub64.p;
         }
-        // The capture lives in s->rf or a caller buffer; the graph bakes the
-        // pointer, so rebuild it when the input pointer changes.
-        if (!s->plain_graph || s->graph_rf != p.rf || s->graph_rf32 != p.rf_f32) {
-            if (s->plain_graph) { cudaGraphExecDestroy(s->plain_graph); s->plain_graph = nullptr; }
-            cudaStream_t cs;
-            ck(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream");
-            cudaGraph_t g;
-            ck(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
-            cudaError_t le = launch_demod_fp64_block(p, cs);
-            cudaError_t ce = cudaStreamEndCapture(cs, &g);
-            cudaStreamDestroy(cs);
-            ck(le, "plain launch");
-            ck(ce, "end capture");
-            ck(cudaGraphInstantiate(&s->plain_graph, g, 0), "graph instantiate");
-            cudaGraphDestroy(g);
-            s->graph_rf = p.rf;
-            s->graph_rf32 = p.rf_f32;
+        // batches of equal size
+        const int64_t batches = (nblocks + kPlainBatch - 1) / kPlainBatch;
+        for (int64_t k = 0; k < batches; k++) {
+            p.first_block = nblocks * k / batches;
+            p.nblocks = (int)(nblocks * (k + 1) / batches - p.first_block);
+            ck(launch_demod_fp64(p, s->stream), "plain launch");
         }
-        int64_t zero = 0;
-        ck(cudaMemcpyAsync(s->pblk.p, &zero, sizeof(int64_t), cudaMemcpyHostToDevice, s->stream), "blk");
-        for (int64_t b = 0; b < nblocks; b++) ck(cudaGraphLaunch(s->plain_graph, s->stream), "graph launch");
+        s->launches += (uint32_t)(batches * (kPlainKernels + (s->sub64.p ? kPlainSubKernels : 0)));
     }
 }
 
@@ -1374,7 +1363,7 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     }
 }
 
-// FP64 plain decode: whole capture, one block per graph replay, then the
+// FP64 plain decode: whole capture in batches of blocks, then the
 // whole-stream pulse scan, the control plane and the field stage in order.
 void decode_plain(vhsdecode_gb300_session* s, const int16_t* rf_dev, uint64_t n, bool demod_only,
                   uint32_t max_fields, uint32_t& stop, double& host_ms, float& demod_ms,
@@ -1388,7 +1377,6 @@ void decode_plain(vhsdecode_gb300_session* s, const int16_t* rf_dev, uint64_t n,
     }
     ck(cudaEventRecord(s->ev[1], cs), "event");
     run_demod(s, rf_dev, nblocks);
-    s->launches += (uint32_t)(nblocks * (kPlainBlockKernels + (s->sub64.p ? kPlainSubKernels : 0)));
     s->segments = 1;
     ck(cudaEventRecord(s->ev[2], cs), "event");
     if (!demod_only && nblocks > 0) {

@@ -1,10 +1,18 @@
-// Plain FP64 block demodulator: one 32768-sample block at a time, full-length
-// complex FFTs in global memory (Stockham radix-8, five passes), one kernel
-// per step.  It restates the same per-block math as the fused FP32 kernel
+// Plain FP64 block demodulator: full-length complex FFTs in global memory
+// (Stockham radix-8, five passes), every kernel over a batch of blocks.  It
+// restates the same per-block math as the fused FP32 kernel
 // (Core/Dsp/RfDemodulator.cs:288-918) in binary64 and is the baseline the
-// fused path is measured against.  The session replays the per-block launch
-// sequence from a captured CUDA graph; the block index is read from device
-// memory so one graph serves every block.
+// fused path is measured against.
+//
+// What bounds it is GB300's binary64 pipe (a warp instruction holds an SM's
+// pipe for about 17 cycles): some 270,000 binary64 warp instructions a block,
+// 15 us of the whole chip.  So a batch of blocks fills the chip (one block at
+// a time left it idle: 0.54 ms a block), the twiddles come from a table of the
+// same sincospi values instead of being computed in every butterfly (as much
+// binary64 work as the transforms), the element-wise steps are the loads and
+// stores of the transforms' first and last passes, and a last pass computes
+// only what is kept: bins 0 .. N/2 of a real signal's spectrum, the real part
+// of a real signal's samples.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -24,83 +32,143 @@ __device__ __forceinline__ double2 wN(int k, bool inv) {
     return make_double2(c, inv ? -s : s);
 }
 
-// Stockham radix-8 pass: in -> out, L = N, Ns in {1, 8, 64, 512, 4096}.
-template <bool INV>
-__global__ void k_pass8(const double2* __restrict__ in, double2* __restrict__ out, int Ns) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_twiddles(double2* tw) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < N) tw[k] = wN(k, false);
+}
+
+// What a transform's first pass reads (kSrc) and its last pass writes (kDst).
+enum Src { kPlainSrc, kRf, kAnalytic, kReal, kFilter, kSub };
+enum Dst { kPlainDst, kHalfDst, kRealDst, kStreamDst };
+struct PassIo {
+    const double2* in;         // [block][N] complex (kPlainSrc; the spectrum of kAnalytic, kFilter, kSub)
+    const double* real;        // [block][N] samples (kReal)
+    const int16_t* rf;         // the batch's first block in the capture (kRf)
+    const float* rf32;
+    const double* gain;        // [kHalf] (kAnalytic)
+    const double2* h;          // [kHalf] (kFilter, kSub)
+    double2* out;              // [block][N] complex
+    double* real_out;          // [block][N] real parts (kRealDst), or the batch's first block in the
+    int shift;                 // stitched stream (kStreamDst: samples n = s + kCut + shift)
+};
+
+template <int kSrc>
+__device__ __forceinline__ double2 pass_load(const PassIo& io, int64_t b, int i) {
+    const double2* in = io.in + b * N;
+    if (kSrc == kRf) {
+        const int64_t n = b * kStride + i;
+        return make_double2(io.rf32 ? (double)io.rf32[n] : (double)io.rf[n], 0.0);
+    }
+    if (kSrc == kReal) return make_double2(io.real[b * N + i], 0.0);
+    if (kSrc == kAnalytic) {
+        // analytic spectrum: X * RfVideo * Hilbert / N  (bins > N/2 zero)
+        if (i > H) return make_double2(0.0, 0.0);
+        const double m = i == 0 || i == H ? io.gain[i] / N : 2.0 * io.gain[i] / N;
+        return make_double2(in[i].x * m, in[i].y * m);
+    }
+    if (kSrc == kFilter) {
+        // Hermitian spectrum D * Hfilter for bins 0..N/2 (imaginary parts of the
+        // DC and Nyquist bins dropped, as a c2r inverse does), mirrored above
+        // N/2, scaled 1/N
+        const int kk = i <= H ? i : N - i;
+        double2 v = cmul(in[kk], io.h[kk]);
+        if (kk == 0 || kk == H) v.y = 0.0;
+        if (i > H) v.y = -v.y;
+        return make_double2(v.x / N, v.y / N);
+    }
+    if (kSrc == kSub) {
+        // sub-deemphasis (ApplySubDeemphasisRealCore, Core/Dsp/RfDemodulator.cs:2852-2990),
+        // step 1: one-sided spectrum whose inverse is the analytic signal of
+        // high = irfft(D Video HighPass): x2 for 0 < k < N/2, real part at 0 and
+        // N/2 (what a c2r inverse keeps), zero above; scaled 1/N
+        if (i > H) return make_double2(0.0, 0.0);
+        const double2 v = cmul(in[i], io.h[i]);
+        if (i == 0 || i == H) return make_double2(v.x / N, 0.0);
+        return make_double2(2.0 * v.x / N, 2.0 * v.y / N);
+    }
+    return in[i];
+}
+
+// Stockham radix-8 pass of block blockIdx.y, L = N, Ns in {1, 8, 64, 512, 4096}.
+template <bool INV, int kSrc, int kDst>
+__global__ void __launch_bounds__(128) k_pass8(PassIo io, const double2* __restrict__ tw, int Ns) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t b = blockIdx.y;
     const int R = 8;
     const int nbf = N / R;
     if (j >= nbf) return;
     int k = j & (Ns - 1);
     double2 v[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = in[j + r * nbf];
-    if (Ns > 1) {
+    for (int r = 0; r < R; r++) v[r] = pass_load<kSrc>(io, b, j + r * nbf);
+    if (kSrc == kPlainSrc) {   // a first pass has no twiddles
 #pragma unroll
         for (int r = 1; r < R; r++) {
-            double2 w = wN((k * r * (N / (Ns * R))) & (N - 1), INV);
+            double2 w = tw[(k * r * (N / (Ns * R))) & (N - 1)];
+            if (INV) w.y = -w.y;
             v[r] = cmul(v[r], w);
         }
     }
     dft<R, INV>(v);
     int dst = (j - k) * R + k;
 #pragma unroll
-    for (int r = 0; r < R; r++) out[dst + r * Ns] = v[r];
-}
-
-// a -> b -> a ... five passes; result ends in `b`.
-template <bool INV>
-void fft(double2* a, double2* b, cudaStream_t s) {
-    int ns = 1;
-    double2* src = a;
-    double2* dst = b;
-    for (int pidx = 0; pidx < 5; pidx++) {
-        k_pass8<INV><<<(N / 8 + 255) / 256, 256, 0, s>>>(src, dst, ns);
-        ns *= 8;
-        double2* t = src; src = dst; dst = t;
+    for (int r = 0; r < R; r++) {
+        const int i = dst + r * Ns;
+        if (kDst == kPlainDst) io.out[b * N + i] = v[r];
+        // the last pass: i = j + r N / 8
+        if (kDst == kHalfDst && (r < R / 2 || (r == R / 2 && j == 0))) io.out[b * N + i] = v[r];
+        if (kDst == kRealDst) io.real_out[b * N + i] = v[r].x;
+        if (kDst == kStreamDst) {
+            const int s = i - kCut - io.shift;
+            if (s >= 0 && s < kStride) io.real_out[b * kStride + s] = v[r].x;
+        }
     }
-    // after 5 passes the data is in `src` (== b)
 }
 
+// One transform of `nb` blocks: first pass from io's source, x and y in turn,
+// the last pass to io's destination (the complex result, if any, in y).
+template <bool INV, int kSrc, int kDst>
+void fft(PassIo io, double2* x, double2* y, const double2* tw, int nb, cudaStream_t s) {
+    const dim3 grid(N / 8 / 128, nb);
+    PassIo p = io;
+    p.out = y;
+    k_pass8<INV, kSrc, kPlainDst><<<grid, 128, 0, s>>>(p, tw, 1);
+    p.in = y; p.out = x;
+    k_pass8<INV, kPlainSrc, kPlainDst><<<grid, 128, 0, s>>>(p, tw, 8);
+    p.in = x; p.out = y;
+    k_pass8<INV, kPlainSrc, kPlainDst><<<grid, 128, 0, s>>>(p, tw, 64);
+    p.in = y; p.out = x;
+    k_pass8<INV, kPlainSrc, kPlainDst><<<grid, 128, 0, s>>>(p, tw, 512);
+    p.in = x; p.out = y;
+    k_pass8<INV, kPlainSrc, kDst><<<grid, 128, 0, s>>>(p, tw, 4096);
+}
 
-// int16 capture, or a float one when rf32 is set
-__global__ void k_load(const int16_t* rf, const float* rf32, const int64_t* blk, double2* out) {
+// demod (float polynomial atan2 of the double analytic signal), the block's
+// spike flag and its spike mask (d > diff_max; a warp holds 32 consecutive n)
+__global__ void k_demod(const double2* z, double* d, float fs, double diff_max, int* flag, unsigned* mask) {
     int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    const int64_t i = blk[0] * kStride + n;
-    out[n] = make_double2(rf32 ? (double)rf32[i] : (double)rf[i], 0.0);
-}
-
-// analytic spectrum: X * RfVideo * Hilbert / N  (bins > N/2 zero)
-__global__ void k_analytic_spec(const double2* X, const double* g, double2* Z) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    double m;
-    if (k == 0 || k == H) m = g[k] / N;
-    else if (k < H) m = 2.0 * g[k] / N;
-    else m = 0.0;
-    Z[k] = make_double2(X[k].x * m, X[k].y * m);
-}
-
-// demod (float polynomial atan2 of the double analytic signal) + spike flag
-__global__ void k_demod(const double2* z, double* d, float fs, double diff_max, int* flag) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+    const int64_t b = blockIdx.y;
+    z += b * N;
     double v = 0.0;
     if (n > 0) {
         float th = vhs_atan2((float)z[n].y, (float)z[n].x);
         float tp = vhs_atan2((float)z[n - 1].y, (float)z[n - 1].x);
         v = (double)vhs_freq_diff(th, tp, fs);
     }
-    d[n] = v;
-    if (n >= 20 && n < N - 20 && v > diff_max) atomicOr(flag, 1);
+    d[b * N + n] = v;
+    const unsigned m = __ballot_sync(0xffffffffu, v > diff_max);
+    if ((n & 31) == 0) mask[b * (N / 32) + (n >> 5)] = m;
+    if (n >= 20 && n < N - 20 && v > diff_max) atomicOr(flag + b, 1);
 }
 
 // diff demod (analytic first difference), only when the block has spikes
 __global__ void k_diff_demod(const double2* z, double* dd, float fs, const int* flag) {
-    if (!flag[0]) return;
+    const int64_t blk = blockIdx.y;
+    if (!flag[blk]) return;
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
+    z += blk * N;
+    dd += blk * N;
     double v = 0.0;
     if (n >= 1) {
         double2 a = z[n], b = z[n - 1];
@@ -119,35 +187,40 @@ __global__ void k_diff_demod(const double2* z, double* dd, float fs, const int* 
 
 // ReplaceSpikes (Core/Dsp/RfDemodulator.cs:966-1001) on one warp, spike set
 // taken from the demod before replacement.
-__global__ void k_replace_spikes(double* d, const double* dd, double diff_max, int* flag,
-                                 unsigned* mask) {
-    if (!flag[0]) return;
+__global__ void __launch_bounds__(32) k_replace_spikes(double* d, const double* dd, int* flag,
+                                                       const unsigned* mask) {
+    const int64_t blk = blockIdx.x;
+    if (!flag[blk]) return;
+    d += blk * N;
+    dd += blk * N;
+    mask += blk * (N / 32);
     int lane = threadIdx.x;
-    for (int base = 0; base < N; base += 32) {
-        unsigned m = __ballot_sync(0xffffffffu, d[base + lane] > diff_max);
-        if (lane == 0) mask[base >> 5] = m;
-    }
-    __syncwarp();
-    for (int word = 0; word < N / 32; word++) {
-        unsigned m = mask[word];
-        while (m) {
-            int b = __ffs(m) - 1;
-            m &= m - 1;
-            int i0 = word * 32 + b;
-            int st = max(i0 - 8, 0), en = min(i0 + 30, N - 1);
-            if (st >= en) continue;
-            double mdd = -INFINITY, md = -INFINITY;
-            for (int k = st + lane; k < en; k += 32) { mdd = fmax(mdd, dd[k]); md = fmax(md, d[k]); }
+    for (int base = 0; base < N / 32; base += 32) {
+        const unsigned mine = mask[base + lane];
+        unsigned words = __ballot_sync(0xffffffffu, mine != 0u);
+        while (words) {
+            const int w = __ffs(words) - 1;
+            words &= words - 1;
+            unsigned m = __shfl_sync(0xffffffffu, mine, w);
+            while (m) {
+                int b = __ffs(m) - 1;
+                m &= m - 1;
+                int i0 = (base + w) * 32 + b;
+                int st = max(i0 - 8, 0), en = min(i0 + 30, N - 1);
+                if (st >= en) continue;
+                double mdd = -INFINITY, md = -INFINITY;
+                for (int k = st + lane; k < en; k += 32) { mdd = fmax(mdd, dd[k]); md = fmax(md, d[k]); }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                mdd = fmax(mdd, __shfl_xor_sync(0xffffffffu, mdd, o));
-                md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
+                for (int o = 16; o > 0; o >>= 1) {
+                    mdd = fmax(mdd, __shfl_xor_sync(0xffffffffu, mdd, o));
+                    md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
+                }
+                if (mdd < md) for (int k = st + lane; k < en; k += 32) d[k] = dd[k];
+                __syncwarp();
             }
-            if (mdd < md) for (int k = st + lane; k < en; k += 32) d[k] = dd[k];
-            __syncwarp();
         }
     }
-    if (lane == 0) flag[0] = 0;
+    if (lane == 0) flag[blk] = 0;
 }
 
 // float32 envelope filtfilt (SosFilter.ApplyForwardBackwardFloat32,
@@ -180,8 +253,13 @@ __device__ __forceinline__ EnvAff env_scan_rev(EnvAff v, int lane) {
     return v;
 }
 
+// The kept samples go to the stitched stream (rows lie wholly inside or
+// outside the kept range).
 __global__ void __launch_bounds__(1024) k_envelope(const double2* z, float* work, double* env, float b0,
                                                    float b1, float a1) {
+    z += (int64_t)blockIdx.x * N;
+    work += (int64_t)blockIdx.x * N;
+    env += (int64_t)blockIdx.x * kStride - kCut;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n0 = warp * 1024;
     const float cc = -a1, gk = b1 - a1 * b0;
@@ -226,27 +304,11 @@ __global__ void __launch_bounds__(1024) k_envelope(const double2* z, float* work
         float zz = lane == 31 ? carry : fmaf(na, carry, nb);
         for (int k = 7; k >= 0; k--) {
             float y = yv[row * 8 + k];
-            env[ms + k] = (double)fmaf(b0, y, zz);
+            if (ms >= kCut && ms < kCut + kStride) env[ms + k] = (double)fmaf(b0, y, zz);
             zz = fmaf(cc, zz, gk * y);
         }
         carry = __shfl_sync(0xffffffffu, zz, 0);
     }
-}
-
-// Sub-deemphasis (ApplySubDeemphasisRealCore, Core/Dsp/RfDemodulator.cs:2852-2990),
-// step 1: one-sided spectrum whose inverse is the analytic signal of
-// high = irfft(D Video HighPass): x2 for 0 < k < N/2, real part at 0 and N/2
-// (what a c2r inverse keeps), zero above; scaled 1/N.
-__global__ void k_sub_spec(const double2* D, const double2* g, double2* A) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    double2 v = make_double2(0.0, 0.0);
-    if (k <= H) {
-        v = cmul(D[k], g[k]);
-        if (k == 0 || k == H) v = make_double2(v.x / N, 0.0);
-        else v = make_double2(2.0 * v.x / N, 2.0 * v.y / N);
-    }
-    A[k] = v;
 }
 
 struct Aff64 { double a, b; };
@@ -277,10 +339,9 @@ __device__ __forceinline__ double sub_gain64(double amp, const SubDeemph64& s) {
     return amp;
 }
 
-// Step 2: amp[n] = |a[n]| * 2 / deviation.
+// Sub-deemphasis step 2: amp[n] = |a[n]| * 2 / deviation.
 __global__ void k_sub_mag(const double2* a, double* amp, SubDeemph64 sub) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+    int64_t n = blockIdx.x * blockDim.x + threadIdx.x + (int64_t)blockIdx.y * N;
     amp[n] = hypot(a[n].x, a[n].y) * sub.inv_half_dev;
 }
 
@@ -296,6 +357,8 @@ template <bool BACKWARD>
 __global__ void __launch_bounds__(32) k_sub_filt(const double* in, double* out, SubDeemph64 sub) {
     const int lane = threadIdx.x;
     const int n0 = blockIdx.x * 1024;
+    in += (int64_t)blockIdx.y * N;
+    out += (int64_t)blockIdx.y * N;
     const double cc = -sub.a1, gk = sub.b1 - sub.a1 * sub.b0, b0 = sub.b0;
     double c8 = cc;
 #pragma unroll
@@ -351,89 +414,68 @@ __global__ void __launch_bounds__(32) k_sub_filt(const double* in, double* out, 
     }
 }
 
-// Step 5, elementwise: video[n] -= Re a[n] (1 - map(amp[n])) + Re a[n] static_factor.
-__global__ void k_sub_apply(const double2* a, const double* amp, double2* video, SubDeemph64 sub) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+// Step 5, elementwise, into the stitched stream: video[n] - (Re a[n] (1 - map(amp[n])) + Re a[n] static_factor).
+__global__ void k_sub_apply(const double2* a, const double* amp, const double* video, double* out, SubDeemph64 sub) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= kStride) return;
+    const int64_t n = (int64_t)blockIdx.y * N + s + kCut;
     double h = a[n].x;
     double g = sub_gain64(amp[n], sub);
-    video[n].x -= h * (1.0 - g) + h * sub.static_factor;
+    double v = video[n];
+    v -= h * (1.0 - g) + h * sub.static_factor;
+    out[(int64_t)blockIdx.y * kStride + s] = v;
 }
-
-__global__ void k_real_to_complex(const double* d, double2* out) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    out[n] = make_double2(d[n], 0.0);
-}
-
-// Hermitian spectrum D * Hfilter for bins 0..N/2 (imaginary parts of the DC and
-// Nyquist bins dropped, as a c2r inverse does), mirrored above N/2, scaled 1/N.
-__global__ void k_filter_spec(const double2* D, const double2* h, double2* out) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    int kk = k <= H ? k : N - k;
-    double2 v = cmul(D[kk], h[kk]);
-    if (kk == 0 || kk == H) v.y = 0.0;
-    if (k > H) v.y = -v.y;
-    out[k] = make_double2(v.x / N, v.y / N);
-}
-
-__global__ void k_store(const double2* x, const int64_t* blk, double* out, int shift) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= kStride) return;
-    int n = s + kCut + shift;
-    out[blk[0] * kStride + s] = x[n].x;
-}
-__global__ void k_store_real(const double* x, const int64_t* blk, double* out) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= kStride) return;
-    out[blk[0] * kStride + s] = x[s + kCut];
-}
-__global__ void k_next_block(int64_t* blk) { blk[0] += 1; }
 
 }  // namespace fp64
 
-// Work buffers: work = 4*N double2 (w0..w3), dwork = 4*N double (d, dd, env, scratch)
-cudaError_t launch_demod_fp64_block(const PlainDemodParams& p, cudaStream_t s) {
+cudaError_t make_fp64_twiddles(double2* tw, cudaStream_t s) {
+    fp64::k_twiddles<<<fp64::N / 256, 256, 0, s>>>(tw);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_demod_fp64(const PlainDemodParams& p, cudaStream_t s) {
     using namespace fp64;
-    const int B = 256, G = (N + B - 1) / B;
+    const int nb = p.nblocks;
+    if (nb <= 0) return cudaSuccess;
+    if (nb > 65535) return cudaErrorInvalidValue;
+    const dim3 every(N / 256, nb), kept((kStride + 255) / 256, nb);
+    const size_t all = (size_t)nb * N;
     double2* w0 = p.work;
-    double2* w1 = p.work + N;
-    double2* w2 = p.work + 2 * N;
-    double2* w3 = p.work + 3 * N;
+    double2* w1 = p.work + all;
+    double2* w2 = p.work + 2 * all;
     double* d = p.dwork;
-    double* dd = p.dwork + N;
-    double* env = p.dwork + 2 * N;
-    float* fscr = p.fwork;
-    int* flag = p.flag;
-    unsigned* mask = p.mask;
-    int64_t* blk = p.blk;
-    k_load<<<G, B, 0, s>>>(p.rf, p.rf_f32, blk, w0);
-    fft<false>(w0, w1, s);                         // X in w1
-    k_analytic_spec<<<G, B, 0, s>>>(w1, p.rf_video, w2);
-    fft<true>(w2, w3, s);                          // z in w3
-    k_demod<<<G, B, 0, s>>>(w3, d, (float)p.fs, p.diff_max, flag);
-    k_diff_demod<<<G, B, 0, s>>>(w3, dd, (float)p.fs, flag);
-    k_replace_spikes<<<1, 32, 0, s>>>(d, dd, p.diff_max, flag, mask);
-    k_envelope<<<1, 1024, 0, s>>>(w3, fscr, env, (float)p.env_b0, (float)p.env_b1, (float)p.env_a1);
-    k_real_to_complex<<<G, B, 0, s>>>(d, w0);
-    fft<false>(w0, w1, s);                         // D in w1
-    k_filter_spec<<<G, B, 0, s>>>(w1, p.video, w2);
-    fft<true>(w2, w3, s);                          // video in w3
+    double* dd = p.dwork + all;
+    double* video = p.dwork + 2 * all;
+    const int64_t first = p.first_block * kStride;
+    PassIo io{};
+    io.rf = p.rf ? p.rf + first : nullptr;
+    io.rf32 = p.rf_f32 ? p.rf_f32 + first : nullptr;
+    fft<false, kRf, kHalfDst>(io, w1, w0, p.twiddle, nb, s);           // X in w0
+    io.in = w0;
+    io.gain = p.rf_video;
+    fft<true, kAnalytic, kPlainDst>(io, w2, w1, p.twiddle, nb, s);     // z in w1
+    k_demod<<<every, 256, 0, s>>>(w1, d, (float)p.fs, p.diff_max, p.flag, p.mask);
+    k_diff_demod<<<every, 256, 0, s>>>(w1, dd, (float)p.fs, p.flag);
+    k_replace_spikes<<<nb, 32, 0, s>>>(d, dd, p.flag, p.mask);
+    k_envelope<<<nb, 1024, 0, s>>>(w1, p.fwork, p.env_out + first, (float)p.env_b0, (float)p.env_b1, (float)p.env_a1);
+    io.real = d;
+    fft<false, kReal, kHalfDst>(io, w1, w0, p.twiddle, nb, s);         // D in w0
+    io.h = p.video;
+    io.real_out = p.sub.high ? video : p.video_out + first;
+    if (p.sub.high) fft<true, kFilter, kRealDst>(io, w2, w1, p.twiddle, nb, s);
+    else fft<true, kFilter, kStreamDst>(io, w2, w1, p.twiddle, nb, s);
     if (p.sub.high) {
-        k_sub_spec<<<G, B, 0, s>>>(w1, p.sub.high, w2);
-        fft<true>(w2, w0, s);                      // analytic high part in w0
-        k_sub_mag<<<G, B, 0, s>>>(w0, dd, p.sub);
-        k_sub_filt<false><<<N / 1024, 32, 0, s>>>(dd, d, p.sub);
-        k_sub_filt<true><<<N / 1024, 32, 0, s>>>(d, dd, p.sub);
-        k_sub_apply<<<G, B, 0, s>>>(w0, dd, w3, p.sub);
+        io.h = p.sub.high;
+        fft<true, kSub, kPlainDst>(io, w2, w1, p.twiddle, nb, s);      // analytic high part in w1
+        k_sub_mag<<<every, 256, 0, s>>>(w1, dd, p.sub);
+        k_sub_filt<false><<<dim3(N / 1024, nb), 32, 0, s>>>(dd, d, p.sub);
+        k_sub_filt<true><<<dim3(N / 1024, nb), 32, 0, s>>>(d, dd, p.sub);
+        k_sub_apply<<<kept, 256, 0, s>>>(w1, dd, video, p.video_out + first, p.sub);
     }
-    k_store<<<(kStride + B - 1) / B, B, 0, s>>>(w3, blk, p.video_out, 0);
-    k_filter_spec<<<G, B, 0, s>>>(w1, p.sync, w2);
-    fft<true>(w2, w0, s);                          // sync in w0
-    k_store<<<(kStride + B - 1) / B, B, 0, s>>>(w0, blk, p.sync_out, 32);
-    k_store_real<<<(kStride + B - 1) / B, B, 0, s>>>(env, blk, p.env_out);
-    k_next_block<<<1, 1, 0, s>>>(blk);
+    io.h = p.sync;
+    io.real_out = p.sync_out + first;
+    io.shift = 32;
+    fft<true, kFilter, kStreamDst>(io, w2, w1, p.twiddle, nb, s);
     return cudaGetLastError();
 }
 

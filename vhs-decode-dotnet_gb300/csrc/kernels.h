@@ -94,7 +94,9 @@ cudaError_t launch_decimate_half(const int16_t* src16, const float* src32, int64
 struct PlainDemodParams {
     const int16_t* rf;
     const float* rf_f32;       // float capture, read instead of rf when set
-    int64_t block;             // block index
+    int64_t first_block;       // the batch: blocks [first_block, first_block + nblocks)
+    int nblocks;
+    const double2* twiddle;    // [32768] exp(-2 pi i k / 32768) (make_fp64_twiddles)
     const double* rf_video;    // [kHalf]
     const double2* video;      // [kHalf]
     const double2* sync;       // [kHalf]
@@ -103,17 +105,21 @@ struct PlainDemodParams {
     double* video_out;         // stitched stream (double)
     double* sync_out;
     double* env_out;
-    double2* work;             // per-block workspace: 4 * 32768 double2
-    double* dwork;             // per-block workspace: 3 * 32768 double
-    float* fwork;              // 32768 + 12 floats (envelope)
-    int* flag;                 // spike flag
-    unsigned* mask;            // 1024 words
-    int64_t* blk;              // device-resident block index, advanced per replay
+    // workspace of nblocks blocks
+    double2* work;             // 3 * 32768 double2 a block
+    double* dwork;             // 3 * 32768 double a block
+    float* fwork;              // 32768 floats a block (envelope)
+    int* flag;                 // spike flag of each block, zero between batches
+    unsigned* mask;            // 1024 words a block
     SubDeemph64 sub;           // sub-deemphasis (sub.high == nullptr: off)
 };
-cudaError_t launch_demod_fp64_block(const PlainDemodParams& p, cudaStream_t stream);
-constexpr int kPlainBlockKernels = 38;  // kernels in one plain-path block (13 + 5 FFTs x 5 passes)
-constexpr int kPlainSubKernels = 10;    // added by sub-deemphasis (5 + 1 FFT x 5 passes)
+// Blocks of one batch: enough to fill the chip (a pass of 128 blocks is 4096
+// CTAs of 128 threads) and to make the launches' gaps small beside it.
+constexpr int kPlainBatch = 128;
+cudaError_t make_fp64_twiddles(double2* tw, cudaStream_t stream);
+cudaError_t launch_demod_fp64(const PlainDemodParams& p, cudaStream_t stream);
+constexpr int kPlainKernels = 29;       // kernels of one batch (4 + 5 FFTs x 5 passes)
+constexpr int kPlainSubKernels = 9;     // added by sub-deemphasis (4 + 1 FFT x 5 passes)
 
 // ---------------------------------------------------------------- pulses
 // Sync-pulse edge events of PulseDetection.FindPulses over a whole stitched

@@ -163,10 +163,7 @@ struct vhsdecode_gb300_session {
     DevBuf<float> pfwork;
     DevBuf<int> pflag;
     DevBuf<unsigned> pmask;
-    DevBuf<int64_t> pblk;
-    cudaGraphExec_t plain_graph = nullptr;
-    const int16_t* graph_rf = nullptr;   // input pointers baked into plain_graph
-    const float* graph_rf32 = nullptr;
+    DevBuf<double2> ptwiddle;
     DevBuf<int64_t> pc_counts, pc_offsets, pc_events, pc_total;
     DevBuf<int64_t> pc_counts_alt, pc_offsets_alt;   // scan scratch of odd segments
     int64_t pc_capacity = 0;
