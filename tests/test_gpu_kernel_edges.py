@@ -96,3 +96,30 @@ def test_fp64_batches(gpu, tape, nblocks):
                     assert np.array_equal(got[c], one.stream(c, 0, STRIDE)), (b, c)
             want = demod.demod_stream(rf, filt, 40e6, dmax, b, 1)
             assert np.max(np.abs(got[0] - want[0])) < 1.0 and np.max(np.abs(got[1] - want[1])) < 1.0, b
+
+
+@pytest.mark.parametrize("blocksize,kind", [(4096, "spikes"), (192, "spikes"), (4608, "noise"), (256, "mixed"),
+                                            (16, "noise"), (1152, "quiet")])
+def test_flac_frames_lossless(gpu, blocksize, kind):
+    # four lanes a frame, eight frames a warp: codes far longer than the bits a
+    # lane holds (a spike of 60000 in a silent partition is a 60000-bit run of
+    # zeros), every predictor order beside constant and verbatim frames in one
+    # warp, blocks shorter than a predictor, a short last frame
+    from vhsd_gb300 import ldf, native
+    rng = np.random.default_rng(blocksize)
+    n = 24 * blocksize + 7
+    x = np.zeros(n, np.int64)
+    if kind == "noise":
+        x = rng.integers(-32768, 32768, n)
+    elif kind == "quiet":
+        x = rng.integers(-1, 2, n)
+    else:
+        at = rng.integers(0, n, n // 150)
+        x[at] = rng.integers(-32768, 32768, len(at))
+    if kind == "mixed":
+        t = np.arange(n)
+        wave = (9000 * np.sin(t * 0.9) + 6000 * np.sin(t * 0.11) + rng.normal(0, 30, n)).astype(np.int64)
+        frame = t // blocksize
+        x = np.where(frame % 4 == 0, x, np.where(frame % 4 == 1, wave, np.where(frame % 4 == 2, 77, wave // 16)))
+    x = x.astype(np.int16)
+    assert np.array_equal(native.flac_decode(ldf.write(x, blocksize=blocksize, seed=blocksize)), x)

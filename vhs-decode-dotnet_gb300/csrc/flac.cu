@@ -8,18 +8,26 @@
 //
 // * k_flac_sync scans every byte position of a chunk for a frame header
 //   (the 14-bit sync code, valid field codes, a valid coded frame or sample
-//   number and a matching CRC-8) and appends the candidates;
+//   number and a matching CRC-8) and appends what it parsed;
 // * the host sorts the candidates and chains them: a frame is accepted where
 //   its number continues the stream's sequence, so a sync pattern inside
-//   compressed data (which also needs a matching CRC-8) is skipped;
-// * k_flac_frames decodes each frame on its own thread (the residual is a
+//   compressed data (which also needs a matching CRC-8) is skipped.  It looks
+//   at no byte of the stream: parsing the headers again and sorting the frames
+//   by a byte of each cost 2.1 ms of cache misses for 10,000 frames;
+// * k_flac_frames decodes each frame with four lanes.  The residual is a
 //   bit-serial Rice code and the prediction a recurrence, so a frame is
-//   sequential work; captures have thousands of frames per second of RF):
-//   each residual value is read and predicted at once, the predictor's
-//   coefficients and history held in registers (one code path per predictor
-//   order), frames handed to threads sorted by subframe type so a warp's lanes
-//   run the same path; it checks that the subframe ends where the next frame
-//   begins and that the frame's CRC-16 matches, and writes int16 samples.
+//   sequential work: what bounds it is the latency of a step, about 120
+//   dependent instructions.  All four lanes read the residual (the same words
+//   of the group's ring); the predictor runs in transposed form, its taps and
+//   partial sums split over the lanes' registers, so a sample costs a lane an
+//   eighth of the 32 multiply-adds at most, no history shifts and one
+//   broadcast.  Frames are handed out sorted by subframe type so a warp's
+//   eight run the same path.  It checks that the subframe ends where the next
+//   frame begins and writes int16 samples (10,000 frames of 4096 samples 1.56
+//   ms, 977 frames 1.1; with a thread a frame, history and CRC in it, 3.9 and
+//   3.6);
+// * k_flac_crc checks the frames' CRC-16, a warp per frame: each lane the
+//   remainder of its 1/32 of the bytes, joined by multiplying with powers of x.
 //
 // Only what RF captures use is accepted: one channel of 16 bits per sample.
 #include <cuda_runtime.h>
@@ -41,74 +49,136 @@
 using namespace vhsd::detail;
 
 namespace vhsd {
+
+// A frame header k_flac_sync found.
+struct FlacCand {
+    int64_t at;
+    uint64_t number;      // coded frame or (variable) sample number
+    int32_t block;
+    int16_t header_len;
+    uint8_t type;         // subframe type bits of the byte after the header
+    bool variable : 1;
+    bool other : 1;       // not one channel of 16 bits
+};
+
 namespace {
 
 __device__ __forceinline__ uint32_t bswap32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
 
-// MSB-first bit reader over 32-bit big-endian words; loads never pass `limit`
-// (a word index): bits beyond it read as zero, and overrun() tells whether any
-// were consumed (the refill looks up to 64 bits ahead, which alone is not an
-// overrun).
+constexpr int kGroup = 4;          // lanes of a frame
+constexpr int kRing = 64;          // words of a frame's ring in shared memory
+constexpr int kAhead = 16;         // words of it that a step outside the top-ups leaves
+constexpr unsigned kWarp = 0xffffffffu;
+
+// MSB-first bit reader over 32-bit big-endian words, by the four lanes of a
+// group together.  Three words wait in registers, the first `bit` bits of the
+// first consumed: the next 32 bits are one funnel shift and a step consumes at
+// most 32.  The words behind them come from a ring in shared memory that the
+// group tops up eight words at a time (two a lane, loaded from global memory
+// one top-up before they enter the ring), at steps the whole warp takes
+// together: a load of its own for every word made the warp wait for the
+// latest load of any of its groups at every step.  A top-up every eight
+// residual values, of a word at most each, keeps the ring ahead.  Loads never pass `limit`
+// (words from the start): bits beyond it read as zero, and overrun() tells
+// whether any were consumed.
 struct BitReader {
-    const uint32_t* w;
-    int64_t next, limit;
-    uint64_t cache;
-    int avail;
-    __device__ void init(const uint32_t* words, int64_t byte_off, int64_t byte_limit) {
-        w = words;
-        next = byte_off >> 2;
-        limit = (byte_limit + 3) >> 2;
-        cache = 0;
-        avail = 0;
-        refill();
-        const int skip = (int)(byte_off & 3) * 8;
-        cache <<= skip;
-        avail -= skip;
+    const uint32_t* w;      // the word the reader started in
+    uint32_t* ring;
+    int lane, limit;
+    int next, filled;       // index of the word after w2; words in the ring
+    int bit;                // 0 .. 31
+    uint32_t w0, w1, w2;
+    unsigned group;         // the group's lanes
+    uint2 pending;          // this lane's words filled + 2 lane, + 1
+    __device__ __forceinline__ uint32_t word(int i) const { return i < limit ? bswap32(__ldg(w + i)) : 0u; }
+    __device__ __forceinline__ void load_pending() {
+        pending = make_uint2(word(filled + 2 * lane), word(filled + 2 * lane + 1));
     }
+    __device__ __forceinline__ void init(const uint32_t* words, int64_t byte_off, int64_t byte_limit, uint32_t* ring_,
+                                         int lane_, unsigned group_) {
+        w = words + (byte_off >> 2);
+        limit = (int)(((byte_limit + 3) >> 2) - (byte_off >> 2));
+        ring = ring_;
+        lane = lane_;
+        group = group_;
+        seek(0, (int)(byte_off & 3) * 8);
+    }
+    __device__ __forceinline__ void push_pending() {
+        *reinterpret_cast<uint2*>(ring + ((filled + 2 * lane) & (kRing - 1))) = pending;
+        filled += 2 * kGroup;
+        load_pending();
+    }
+    // the ring from word `next` on, at least kAhead words of it
     __device__ __forceinline__ void refill() {
-        while (avail <= 32) {
-            uint32_t v = 0;
-            if (next < limit) v = bswap32(__ldg(w + next));
+        __syncwarp(group);
+        filled = next & ~1;
+        load_pending();
+        push_pending();
+        push_pending();
+        push_pending();
+        __syncwarp(group);
+    }
+    __device__ __forceinline__ void seek(int i, int bit_) {   // to bit `bit_` of word i
+        bit = bit_;
+        w0 = word(i);
+        w1 = word(i + 1);
+        w2 = word(i + 2);
+        next = i + 3;
+        refill();
+    }
+    // eight words more if there is room (by whole warps, at steps they take
+    // together)
+    __device__ __forceinline__ void top_up() {
+        __syncwarp();
+        if (filled - next <= kRing - 8) push_pending();
+        __syncwarp();
+    }
+    __device__ __forceinline__ uint32_t top() const { return __funnelshift_l(w1, w0, bit); }
+    // consumes 0 <= n <= 32 bits; the ring holds the next word
+    __device__ __forceinline__ void skip_fast(int n) {
+        bit += n;
+        if (bit >= 32) {
+            bit -= 32;
+            w0 = w1;
+            w1 = w2;
+            w2 = ring[next & (kRing - 1)];
             next++;
-            cache |= (uint64_t)v << (32 - avail);
-            avail += 32;
         }
     }
+    // the same from anywhere: leaves kAhead words in the ring
+    __device__ __forceinline__ void skip(int n) {
+        skip_fast(n);
+        if (filled - next < kAhead) refill();
+    }
     __device__ __forceinline__ uint32_t get(int n) {   // 0 <= n <= 32
-        if (n == 0) return 0;
-        if (avail < n) refill();
-        uint32_t v = (uint32_t)(cache >> (64 - n));
-        cache <<= n;
-        avail -= n;
+        const uint32_t v = n == 0 ? 0u : top() >> (32 - n);
+        skip(n);
         return v;
     }
     __device__ __forceinline__ int32_t sget(int n) {
         if (n == 0) return 0;
-        uint32_t v = get(n);
+        const uint32_t v = get(n);
         return (int32_t)(v << (32 - n)) >> (32 - n);
     }
     // zeros before the next one bit (the bit is consumed); -1 past `cap` zeros
     __device__ __forceinline__ int32_t unary(int32_t cap) {
         int32_t q = 0;
         for (;;) {
-            if (avail < 32) refill();
-            const uint32_t top = (uint32_t)(cache >> 32);
-            if (top) {
-                const int z = __clz(top);
-                cache <<= (z + 1);
-                avail -= z + 1;
+            const uint32_t t = top();
+            if (t) {
+                const int z = __clz(t);
+                skip(z + 1);
                 q += z;
                 return q <= cap ? q : -1;
             }
-            cache <<= 32;
-            avail -= 32;
+            skip(32);
             q += 32;
             if (q > cap || overrun()) return -1;
         }
     }
-    // bit position relative to the word array
-    __device__ __forceinline__ int64_t bitpos() const { return next * 32 - avail; }
-    __device__ __forceinline__ bool overrun() const { return bitpos() > limit * 32; }
+    // bits from the start of the reader's first word
+    __device__ __forceinline__ int64_t bitpos() const { return (int64_t)(next - 3) * 32 + bit; }
+    __device__ __forceinline__ bool overrun() const { return bitpos() > (int64_t)limit * 32; }
 };
 
 __device__ __forceinline__ bool utf8_number(const uint8_t* p, int64_t n, int64_t at, int& len, uint64_t& val) {
@@ -177,15 +247,19 @@ __device__ int parse_header(const uint8_t* p, int64_t n, int64_t at, uint64_t& n
 }
 
 // Candidate frame headers: one thread per byte position.
-__global__ void k_flac_sync(const uint8_t* __restrict__ p, int64_t n, int64_t* cand, int* count, int cap) {
+__global__ void k_flac_sync(const uint8_t* __restrict__ p, int64_t n, FlacCand* cand, int* count, int cap) {
     const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (at + 1 >= n || p[at] != 0xFF || (p[at + 1] & 0xFE) != 0xF8) return;
-    uint64_t num;
-    int block;
+    FlacCand c{};
     bool var;
-    if (!parse_header(p, n, at, num, block, var)) return;
+    c.header_len = parse_header(p, n, at, c.number, c.block, var);
+    if (!c.header_len) return;
+    c.at = at;
+    c.variable = var;
+    c.other = (p[at + 3] >> 4) != 0 || ((p[at + 3] >> 1) & 7) != 4;
+    c.type = p[at + c.header_len] & 0x7E;   // the buffer is padded
     const int k = atomicAdd(count, 1);
-    if (k < cap) cand[k] = at;
+    if (k < cap) cand[k] = c;
 }
 
 // Residual of a subframe (RFC 9639 section 9.2.7), read one value at a time:
@@ -194,7 +268,7 @@ __global__ void k_flac_sync(const uint8_t* __restrict__ p, int64_t n, int64_t* c
 struct Residual {
     int pbits, esc, porder, part, parts, left, k, width, order, block;
     bool escaped;
-    __device__ int init(BitReader& r, int block_, int order_) {
+    __device__ __forceinline__ int init(BitReader& r, int block_, int order_) {
         block = block_;
         order = order_;
         const int method = (int)r.get(2);
@@ -223,185 +297,265 @@ struct Residual {
             v = r.sget(width);
             return true;
         }
-        const int32_t q = r.unary(1 << 20);
-        if (q < 0) return false;
-        const uint32_t u = ((uint32_t)q << k) | r.get(k);
+        const uint32_t top = r.top();
+        const int z = __clz(top), len = z + 1 + k;
+        uint32_t u;
+        if (len <= 32) {
+            // the whole code lies in the next 32 bits: z zeros, a one, k bits
+            // (two shifts: k = 0 shifts everything out, z = 31 the one)
+            u = (uint32_t)z << k | top << z << 1 >> 1 >> (31 - k);
+            r.skip_fast(len);
+        } else {
+            const int32_t q = r.unary(1 << 20);
+            if (q < 0) return false;
+            u = ((uint32_t)q << k) | r.get(k);
+        }
         v = (int32_t)(u >> 1) ^ -(int32_t)(u & 1);
         return true;
     }
 };
 
-// Output of one frame's samples: four int16 packed per 8-byte store when the
-// frame's first sample is 8-byte aligned (a thread's stores go to its own
-// frame, so a warp's scalar stores would touch 32 lines each).
-struct Out4 {
-    int16_t* o;
-    uint64_t a;
-    int i, n;
-    bool vec;
-    __device__ void init(int16_t* o_) {
-        o = o_;
-        a = 0;
-        i = n = 0;
-        vec = ((uintptr_t)o_ & 7) == 0;
+// Output of one frame's samples by its four lanes: lane l keeps sample 4 m + l,
+// and every fourth sample the group stores eight bytes side by side.
+struct GroupOut {
+    int16_t* o;   // this lane's next sample
+    int i, lane;
+    int16_t mine;
+    __device__ __forceinline__ void init(int16_t* out, int lane_) {
+        o = out + lane_;
+        i = 0;
+        lane = lane_;
+        mine = 0;
     }
-    __device__ __forceinline__ void put(int32_t x) {
-        if (!vec) {
-            o[i++] = (int16_t)x;
-            return;
-        }
-        a = (a >> 16) | ((uint64_t)(uint16_t)x << 48);
-        i++;
-        if (++n == 4) {
-            *reinterpret_cast<uint64_t*>(o + i - 4) = a;
-            n = 0;
+    __device__ __forceinline__ void put(int32_t x) {   // by every lane of the group
+        if (i == lane) mine = (int16_t)x;
+        i = (i + 1) & (kGroup - 1);
+        if (i == 0) {
+            *o = mine;
+            o += kGroup;
         }
     }
     __device__ __forceinline__ void flush() {
-        for (int k = 0; k < n; k++) o[i - n + k] = (int16_t)(a >> (16 * (4 - n + k)));
-        n = 0;
+        if (lane < i) *o = mine;
     }
 };
 
-// Fixed predictor of order O (RFC 9639 section 9.2.5), history in registers.
-template <int O>
-__device__ int fixed_subframe(BitReader& r, int block, int bps, int wasted, Out4& o) {
-    int32_t h[O > 0 ? O : 1];   // h[0]: the latest sample
+// What a group knows of its predicted subframe (RFC 9639 sections 9.2.5,
+// 9.2.6) before its samples.
+struct Predicted {
+    bool active;      // the frame has a predicted subframe and no error so far
+    bool fixed;
+    int order, block, bps, wasted;
+};
+
+// The samples of the predicted subframes of a warp's eight frames, of order
+// <= 4 T, the group's lane l holding taps [T l, T l + T) in transposed form:
+// s[t] is the sum, over the samples so far, of the products that the sample
+// T l + t steps ahead will be predicted from (tap j of sample x goes into the
+// sum of the sample j + 1 steps after it), accumulated in 64 bits.  The fixed
+// predictors are the same with whole-number taps and no shift.  The whole warp
+// takes every step together (a group that has ended or failed idles): with the
+// groups on their own the shuffles of one group at a time ran the eight frames
+// one after the other.  Returns the group's error.
+template <int T>
+__device__ __forceinline__ int predicted_samples(BitReader& r, Predicted f, int lane, GroupOut& o) {
+    int err = 0;
+    bool on = f.active;
+    const int warm_word = r.next - 3, warm_bit = r.bit;   // the warm-up samples, read again once the taps are known
+    int32_t c[T];
 #pragma unroll
-    for (int j = O - 1; j >= 0; j--) {
-        h[j] = r.sget(bps);
-        o.put(h[j] << wasted);
-    }
+    for (int t = 0; t < T; t++) c[t] = 0;
+    int shift = 0;
     Residual res;
-    if (int e = res.init(r, block, O)) return e;
-    for (int i = O; i < block; i++) {
-        int32_t e;
-        if (!res.next(r, e)) return 5;
-        int32_t x = e;
-        if (O == 1) x += h[0];
-        if (O == 2) x += 2 * h[0] - h[1];
-        if (O == 3) x += 3 * h[0] - 3 * h[1] + h[2];
-        if (O == 4) x += 4 * h[0] - 6 * h[1] + 4 * h[2] - h[3];
+    if (on) {
+        for (int i = 0; i < f.order; i++) r.get(f.bps);
+        if (f.fixed) {
+            // taps of x[i-1], x[i-2], ...: 1; 2, -1; 3, -3, 1; 4, -6, 4, -1
+            const int n = f.order;
+            const int32_t tap[4] = {n, n == 1 ? 0 : n == 2 ? -1 : n == 3 ? -3 : n == 4 ? -6 : 0,
+                                    n == 3 ? 1 : n == 4 ? 4 : 0, n == 4 ? -1 : 0};
 #pragma unroll
-        for (int j = O - 1; j > 0; j--) h[j] = h[j - 1];
-        if (O > 0) h[0] = x;
-        o.put(x << wasted);
+            for (int j = 0; j < 4; j++)
+                if (lane == j / T) c[j % T] = tap[j];
+        } else {
+            const int prec = (int)r.get(4) + 1;
+            shift = r.sget(5);
+            if (prec == 16) err = 6;
+            else if (shift < 0) err = 7;
+            if (!err)
+#pragma unroll
+                for (int j = 0; j < kGroup * T; j++)
+                    if (j < f.order) {
+                        const int32_t v = r.sget(prec);
+                        if (lane == j / T) c[j % T] = v;
+                    }
+        }
+        if (!err) err = res.init(r, f.block, f.order);
+        if (err) on = false;
     }
-    return 0;
+    int64_t s[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) s[t] = 0;
+    // the sums move one sample on: the next lane's nearest sum (before x)
+    // enters this lane's farthest slot
+    auto next_sum = [&]() -> int64_t {
+        const uint32_t lo = __shfl_down_sync(kWarp, (uint32_t)s[0], 1, kGroup);
+        const uint32_t hi = __shfl_down_sync(kWarp, (uint32_t)((uint64_t)s[0] >> 32), 1, kGroup);
+        return lane == kGroup - 1 ? 0 : (int64_t)((uint64_t)hi << 32 | lo);
+    };
+    auto feed = [&](int32_t x, int64_t from) {
+#pragma unroll
+        for (int t = 0; t < T; t++) s[t] = (t + 1 < T ? s[t + 1] : from) + (int64_t)c[t] * x;
+    };
+    const int res_word = r.next - 3, res_bit = r.bit;
+    r.seek(warm_word, warm_bit);
+    const int warm_steps = __reduce_max_sync(kWarp, on ? f.order : 0);
+    for (int i = 0; i < warm_steps; i++) {
+        const int64_t from = next_sum();
+        if (on && i < f.order) {
+            const int32_t x = r.sget(f.bps);
+            feed(x, from);
+            o.put(x << f.wasted);
+        }
+    }
+    r.seek(res_word, res_bit);
+    int n = on ? f.block - f.order : 0;
+    const int steps = __reduce_max_sync(kWarp, n);
+    for (int i = 0; i < steps; i++) {
+        if ((i & 7) == 0) r.top_up();   // a step takes a word at most, save for very long codes
+        const int64_t from = next_sum();
+        const int32_t ahead = __shfl_sync(kWarp, (int32_t)__funnelshift_r((uint32_t)s[0], (uint32_t)((uint64_t)s[0] >> 32), shift), 0, kGroup);
+        if (i < n) {
+            int32_t e;
+            if (res.next(r, e)) {
+                const int32_t x = e + ahead;
+                feed(x, from);
+                o.put(x << f.wasted);
+            } else {
+                err = 5;
+                n = 0;
+            }
+        }
+    }
+    return err;
 }
 
-// Linear predictor of order P (RFC 9639 section 9.2.6): coefficients and
-// history in registers, products accumulated in 64 bits.
-template <int P>
-__device__ int lpc_subframe(BitReader& r, int block, int bps, int wasted, Out4& o) {
-    int32_t h[P];
-#pragma unroll
-    for (int j = P - 1; j >= 0; j--) {
-        h[j] = r.sget(bps);
-        o.put(h[j] << wasted);
+// Four lanes per frame, frames taken in the order `order_idx` gives (sorted by
+// subframe type, so the groups of a warp run the same predictor).  Every lane
+// of a group reads the same bits and takes the same branches.
+__global__ void __launch_bounds__(64) k_flac_frames(const uint32_t* __restrict__ words, const FlacFrame* frames,
+                                                    const int* order_idx, int nframes, int16_t* out, int* status) {
+    __shared__ __align__(8) uint32_t rings[64 / kGroup][kRing];
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+    const bool valid = t < nframes;
+    const int lane = threadIdx.x % kGroup;
+    const int f = order_idx[valid ? t : nframes - 1];
+    const FlacFrame fr = frames[f];
+    GroupOut o;
+    o.init(out + fr.sample0, lane);
+    int err = 0;
+    BitReader r;
+    r.init(words, fr.off + fr.header_len, fr.end, rings[threadIdx.x / kGroup], lane,
+           ((1u << kGroup) - 1) << (threadIdx.x % 32 / kGroup * kGroup));
+    const int block = fr.block;
+    Predicted p{};
+    p.block = block;
+    if (valid) {
+        do {
+            if (r.get(1) != 0) { err = 10; break; }
+            const int type = (int)r.get(6);
+            if (r.get(1)) {
+                const int32_t z = r.unary(15);
+                if (z < 0) { err = 11; break; }
+                p.wasted = z + 1;
+            }
+            p.bps = 16 - p.wasted;
+            if (p.bps <= 0) { err = 12; break; }
+            if (type == 0) {
+                const int32_t v = r.sget(p.bps);
+                for (int i = 0; i < block; i++) o.put(v << p.wasted);
+            } else if (type == 1) {
+                for (int i = 0; i < block; i++) {
+                    const int32_t v = r.sget(p.bps);
+                    o.put(v << p.wasted);
+                }
+            } else if ((type >= 8 && type <= 12) || type >= 32) {
+                p.fixed = type < 32;
+                p.order = p.fixed ? type - 8 : type - 31;
+                if (p.order > block) { err = p.fixed ? 13 : 14; break; }
+                p.active = true;
+            } else {
+                err = 17;
+            }
+        } while (false);
     }
-    const int prec = (int)r.get(4) + 1;
-    if (prec == 16) return 6;
-    const int shift = r.sget(5);
-    if (shift < 0) return 7;
-    int32_t c[P];
-#pragma unroll
-    for (int j = 0; j < P; j++) c[j] = r.sget(prec);
-    Residual res;
-    if (int e = res.init(r, block, P)) return e;
-    for (int i = P; i < block; i++) {
-        int32_t e;
-        if (!res.next(r, e)) return 5;
-        // four partial sums, so the products do not form one dependent chain
-        int64_t acc[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int j = 0; j < P; j++) acc[j & 3] += (int64_t)c[j] * h[j];
-        const int32_t x = e + (int32_t)(((acc[0] + acc[1]) + (acc[2] + acc[3])) >> shift);
-#pragma unroll
-        for (int j = P - 1; j > 0; j--) h[j] = h[j - 1];
-        h[0] = x;
-        o.put(x << wasted);
+    const int most = __reduce_max_sync(kWarp, p.active ? p.order + 1 : 0);   // 0: no predicted frame
+    if (most > 0) {
+        int e;
+        if (most <= kGroup + 1) e = predicted_samples<1>(r, p, lane, o);
+        else if (most <= 2 * kGroup + 1) e = predicted_samples<2>(r, p, lane, o);
+        else if (most <= 4 * kGroup + 1) e = predicted_samples<4>(r, p, lane, o);
+        else e = predicted_samples<8>(r, p, lane, o);
+        if (e) err = (p.fixed ? 20 : 30) + e;
     }
-    return 0;
+    if (valid && !err) {
+        o.flush();
+        const int64_t start = (fr.off + fr.header_len) & ~(int64_t)3;   // the reader's first word
+        if (r.overrun()) err = 18;
+        // byte alignment, then the frame's CRC-16 (k_flac_crc) must end the frame
+        else if (start + ((r.bitpos() + 7) >> 3) + 2 != fr.end) err = 19;
+    }
+    if (valid && err && lane == 0) atomicCAS(status, 0, (f << 8) | err);
 }
 
-template <int P = 1>
-__device__ int lpc_dispatch(int order, BitReader& r, int block, int bps, int wasted, Out4& o) {
-    if constexpr (P > 32) {
-        return 8;
-    } else {
-        if (order == P) return lpc_subframe<P>(r, block, bps, wasted, o);
-        return lpc_dispatch<P + 1>(order, r, block, bps, wasted, o);
+// a b mod x^16 + x^15 + x^2 + 1 over GF(2), the CRC-16's polynomial
+__device__ __forceinline__ uint32_t gf16_mul(uint32_t a, uint32_t b) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 15; i >= 0; i--) {
+        v = v << 1 ^ (v & 0x8000u ? 0x18005u : 0u);
+        if (b >> i & 1) v ^= a;
     }
+    return v & 0xffffu;
 }
 
-// One frame per thread, frames taken in the order `order_idx` gives (sorted
-// by subframe type, so the lanes of a warp run the same predictor).
-__global__ void __launch_bounds__(64, 1) k_flac_frames(const uint32_t* __restrict__ words, const FlacFrame* frames,
-                                                     const int* order_idx, int nframes, int16_t* out, int* status) {
+// The frames' CRC-16, a warp per frame: bytes [off, end - 2) cut into 32 runs
+// of equal length (the first one short), each lane the remainder of its own;
+// two neighbouring remainders join as left x^(8 length of right) + right.
+// A frame that failed already keeps its error.
+__global__ void __launch_bounds__(128) k_flac_crc(const uint8_t* __restrict__ bytes, const FlacFrame* frames,
+                                                  int nframes, int* status) {
     __shared__ uint16_t t16[256];   // per-thread table indices: shared, not constant, memory
     for (int i = threadIdx.x; i < 256; i += blockDim.x) t16[i] = c_crc16[i];
     __syncthreads();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nframes) return;
-    const int f = order_idx[t];
-    const FlacFrame fr = frames[f];
-    const uint8_t* bytes = reinterpret_cast<const uint8_t*>(words);
-    Out4 o;
-    o.init(out + fr.sample0);
-    int err = 0;
-    BitReader r;
-    r.init(words, fr.off + fr.header_len, fr.end);
-    const int block = fr.block;
-    do {
-        if (r.get(1) != 0) { err = 10; break; }
-        const int type = (int)r.get(6);
-        int wasted = 0;
-        if (r.get(1)) {
-            const int32_t z = r.unary(15);
-            if (z < 0) { err = 11; break; }
-            wasted = z + 1;
-        }
-        const int bps = 16 - wasted;
-        if (bps <= 0) { err = 12; break; }
-        if (type == 0) {
-            const int32_t v = r.sget(bps);
-            for (int i = 0; i < block; i++) o.put(v << wasted);
-        } else if (type == 1) {
-            for (int i = 0; i < block; i++) o.put(r.sget(bps) << wasted);
-        } else if (type >= 8 && type <= 12) {
-            const int ord = type - 8;
-            if (ord > block) { err = 13; break; }
-            int e = 0;
-            switch (ord) {
-            case 0: e = fixed_subframe<0>(r, block, bps, wasted, o); break;
-            case 1: e = fixed_subframe<1>(r, block, bps, wasted, o); break;
-            case 2: e = fixed_subframe<2>(r, block, bps, wasted, o); break;
-            case 3: e = fixed_subframe<3>(r, block, bps, wasted, o); break;
-            default: e = fixed_subframe<4>(r, block, bps, wasted, o); break;
-            }
-            if (e) { err = 20 + e; break; }
-        } else if (type >= 32) {
-            const int ord = type - 31;
-            if (ord > block) { err = 14; break; }
-            const int e = lpc_dispatch(ord, r, block, bps, wasted, o);
-            if (e) { err = 30 + e; break; }
-        } else {
-            err = 17;
-            break;
-        }
-        o.flush();
-        if (r.overrun()) { err = 18; break; }
-        // byte alignment, then the frame's CRC-16 must end the frame
-        const int64_t bit = r.bitpos();
-        const int64_t end_byte = (bit + 7) >> 3;
-        if (end_byte + 2 != fr.end) { err = 19; break; }
-        uint16_t crc = 0;
-        for (int64_t i = fr.off; i < end_byte; i++)
-            crc = (uint16_t)((crc << 8) ^ t16[(crc >> 8) ^ bytes[i]]);
-        if (crc != (uint16_t)((bytes[end_byte] << 8) | bytes[end_byte + 1])) { err = 40; break; }
-    } while (false);
-    if (err) atomicCAS(status, 0, (f << 8) | err);
+    const int f = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (f >= nframes) return;
+    const int64_t off = frames[f].off, end = frames[f].end;
+    const int64_t n = end - 2 - off;
+    if (n <= 0) return;   // shorter than any frame: the decoder reports it
+    const int64_t run = (n + 31) / 32, pad = 32 * run - n;
+    const int64_t b = off + max(run * lane - pad, (int64_t)0), e = off + max(run * (lane + 1) - pad, (int64_t)0);
+    uint32_t crc = 0;
+    auto byte = [&](uint32_t v) { crc = (crc << 8 ^ t16[crc >> 8 ^ v]) & 0xffffu; };
+    int64_t i = b;
+    for (; i < e && (i & 3); i++) byte(bytes[i]);
+    for (; i + 4 <= e; i += 4) {   // the buffer is word-aligned
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(bytes + i);
+        byte(w & 0xffu);
+        byte(w >> 8 & 0xffu);
+        byte(w >> 16 & 0xffu);
+        byte(w >> 24);
+    }
+    for (; i < e; i++) byte(bytes[i]);
+    uint32_t x = 1;   // x^(8 run)
+    for (int64_t k = 0; k < run; k++) x = (x << 8 ^ t16[x >> 8]) & 0xffffu;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t right = __shfl_down_sync(0xffffffffu, crc, d);
+        crc = gf16_mul(crc, x) ^ right;   // kept by the lanes that are multiples of 2 d
+        x = gf16_mul(x, x);
+    }
+    if (lane == 0 && crc != ((uint32_t)bytes[end - 2] << 8 | bytes[end - 1])) atomicCAS(status, 0, (f << 8) | 40);
 }
 
 std::vector<uint8_t> make_crc8() {
@@ -421,48 +575,6 @@ std::vector<uint16_t> make_crc16() {
         t[b] = c;
     }
     return t;
-}
-
-// host-side parse of one header (same rules as the device's), for chaining
-int host_header(const uint8_t* p, int64_t n, int64_t at, uint64_t& number, int& block, bool& variable) {
-    if (at + 6 > n || p[at] != 0xFF || (p[at + 1] & 0xFE) != 0xF8) return 0;
-    variable = p[at + 1] & 1;
-    const int bcode = p[at + 2] >> 4, rcode = p[at + 2] & 15;
-    const int chan = p[at + 3] >> 4, scode = (p[at + 3] >> 1) & 7;
-    if (bcode == 0 || rcode == 15 || chan > 10 || scode == 3 || (p[at + 3] & 1)) return 0;
-    uint8_t b0 = p[at + 4];
-    int extra;
-    uint64_t v;
-    if (b0 < 0x80) { extra = 0; v = b0; }
-    else if ((b0 & 0xE0) == 0xC0) { extra = 1; v = b0 & 0x1F; }
-    else if ((b0 & 0xF0) == 0xE0) { extra = 2; v = b0 & 0x0F; }
-    else if ((b0 & 0xF8) == 0xF0) { extra = 3; v = b0 & 0x07; }
-    else if ((b0 & 0xFC) == 0xF8) { extra = 4; v = b0 & 0x03; }
-    else if ((b0 & 0xFE) == 0xFC) { extra = 5; v = b0 & 0x01; }
-    else if (b0 == 0xFE) { extra = 6; v = 0; }
-    else return 0;
-    if (at + 4 + extra >= n) return 0;
-    for (int i = 1; i <= extra; i++) {
-        uint8_t b = p[at + 4 + i];
-        if ((b & 0xC0) != 0x80) return 0;
-        v = (v << 6) | (b & 0x3F);
-    }
-    int64_t q = at + 5 + extra;
-    if (bcode == 6) { if (q + 1 > n) return 0; block = p[q] + 1; q += 1; }
-    else if (bcode == 7) { if (q + 2 > n) return 0; block = ((p[q] << 8) | p[q + 1]) + 1; q += 2; }
-    else if (bcode == 1) block = 192;
-    else if (bcode <= 5) block = 576 << (bcode - 2);
-    else block = 256 << (bcode - 8);
-    if (rcode == 12) q += 1;
-    else if (rcode == 13 || rcode == 14) q += 2;
-    if (q + 1 > n) return 0;
-    static const std::vector<uint8_t> t8 = make_crc8();
-    uint8_t c = 0;
-    for (int64_t i = at; i < q; i++) c = t8[c ^ p[i]];
-    if (c != p[q]) return 0;
-    number = v;
-    if (chan != 0 || scode != 4) return -1;   // a valid header of a format RF captures do not use
-    return (int)(q + 1 - at);
 }
 
 }  // namespace
@@ -526,7 +638,7 @@ void FlacStreamDecoder::reserve(size_t bytes, size_t samples, size_t frames) {
         have = want;
     };
     grow((void**)&d_bytes, cap_bytes, (bytes + 96) & ~(size_t)15);
-    grow((void**)&d_cand, cap_cand, std::max<size_t>(frames, 1024) * sizeof(int64_t));
+    grow((void**)&d_cand, cap_cand, std::max<size_t>(frames, 1024) * sizeof(FlacCand));
     grow((void**)&d_frames, cap_frames, std::max<size_t>(frames + 16, 64) * sizeof(FlacFrame));
     grow((void**)&d_work, cap_work, std::max<size_t>(frames, 1) * sizeof(int32_t));   // frame order
     grow((void**)&d_out, cap_out, std::max<size_t>(samples, 1) * sizeof(int16_t));
@@ -556,7 +668,7 @@ size_t FlacStreamDecoder::decode_to(const uint8_t* p, size_t n, bool at_eof,
     if (timing)
         for (auto& e : ev) ck(cudaEventCreate(&e), "event");
     if (timing) ck(cudaEventRecord(ev[0], stream), "event");
-    const int cap = (int)(cap_cand / sizeof(int64_t));
+    const int cap = (int)(cap_cand / sizeof(FlacCand));
     k_flac_sync<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(d_bytes, (int64_t)n, d_cand, d_misc, cap);
     ck(cudaGetLastError(), "flac sync launch");
     if (timing) ck(cudaEventRecord(ev[1], stream), "event");
@@ -564,22 +676,22 @@ size_t FlacStreamDecoder::decode_to(const uint8_t* p, size_t n, bool at_eof,
     ck(cudaMemcpyAsync(&count, d_misc, sizeof(int), cudaMemcpyDeviceToHost, stream), "d2h");
     ck(cudaStreamSynchronize(stream), "sync");
     if (count > cap) throw Failure(VHSDECODE_GB300_STATUS_INPUT_ERROR, "too many FLAC frame candidates");
-    std::vector<int64_t> cand((size_t)count);
-    if (count) ck(cudaMemcpy(cand.data(), d_cand, (size_t)count * sizeof(int64_t), cudaMemcpyDeviceToHost), "d2h");
-    std::sort(cand.begin(), cand.end());
+    std::vector<FlacCand> cand((size_t)count);
+    if (count) ck(cudaMemcpy(cand.data(), d_cand, (size_t)count * sizeof(FlacCand), cudaMemcpyDeviceToHost), "d2h");
+    std::sort(cand.begin(), cand.end(), [](const FlacCand& a, const FlacCand& b) { return a.at < b.at; });
     // chain: the chunk starts on a frame; accept headers that continue the sequence
     std::vector<FlacFrame> frames;
+    std::vector<uint8_t> types;   // each frame's subframe type byte
+    frames.reserve(cand.size());
+    types.reserve(cand.size());
     int64_t expect_at = 0;
     for (size_t i = 0; i < cand.size(); i++) {
-        const int64_t at = cand[i];
+        const int64_t at = cand[i].at;
         if (at < expect_at) continue;
-        uint64_t num = 0;
-        int block = 0;
-        bool var = false;
-        const int hl = host_header(p, (int64_t)n, at, num, block, var);
-        if (hl == 0) continue;
-        const uint64_t want = var ? next_sample : next_frame;
-        if (hl < 0) {
+        const uint64_t num = cand[i].number;
+        const int block = cand[i].block, hl = cand[i].header_len;
+        const uint64_t want = cand[i].variable ? next_sample : next_frame;
+        if (cand[i].other) {
             // a header of another sample format where this stream's next frame belongs
             if (num == want) throw Failure(VHSDECODE_GB300_STATUS_INPUT_ERROR, "FLAC stream is not 16-bit mono");
             continue;
@@ -598,6 +710,7 @@ size_t FlacStreamDecoder::decode_to(const uint8_t* p, size_t n, bool at_eof,
         fr.block = block;
         fr.sample0 = (int64_t)(next_sample - sample_base);
         frames.push_back(fr);
+        types.push_back(cand[i].type);
         next_frame++;
         next_sample += (uint64_t)block;
         expect_at = at + hl;
@@ -617,17 +730,20 @@ size_t FlacStreamDecoder::decode_to(const uint8_t* p, size_t n, bool at_eof,
     // frames sorted by subframe type (the byte after the frame header), so the
     // lanes of a warp decode with the same predictor
     std::vector<int> idx(frames.size());
-    for (size_t i = 0; i < idx.size(); i++) idx[i] = (int)i;
-    std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
-        return (p[frames[(size_t)a].off + frames[(size_t)a].header_len] & 0x7E) <
-               (p[frames[(size_t)b].off + frames[(size_t)b].header_len] & 0x7E);
-    });
+    {
+        size_t first[257] = {};
+        for (size_t i = 0; i < idx.size(); i++) first[types[i] + 1]++;
+        for (int t = 0; t < 256; t++) first[t + 1] += first[t];
+        for (size_t i = 0; i < idx.size(); i++) idx[first[types[i]]++] = (int)i;
+    }
     ck(cudaMemcpyAsync(d_frames, frames.data(), frames.size() * sizeof(FlacFrame), cudaMemcpyHostToDevice, stream),
        "h2d frames");
     ck(cudaMemcpyAsync(d_work, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, stream), "h2d order");
     if (timing) ck(cudaEventRecord(ev[2], stream), "event");
-    k_flac_frames<<<(unsigned)((frames.size() + 63) / 64), 64, 0, stream>>>(
+    k_flac_frames<<<(unsigned)((frames.size() * kGroup + 63) / 64), 64, 0, stream>>>(
         reinterpret_cast<const uint32_t*>(d_bytes), d_frames, d_work, (int)frames.size(), d_out, d_misc + 1);
+    k_flac_crc<<<(unsigned)((frames.size() + 3) / 4), 128, 0, stream>>>(d_bytes, d_frames, (int)frames.size(),
+                                                                       d_misc + 1);
     if (timing) ck(cudaEventRecord(ev[3], stream), "event");
     ck(cudaGetLastError(), "flac decode launch");
     int st = 0;

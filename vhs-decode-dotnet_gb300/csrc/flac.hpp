@@ -44,7 +44,7 @@ private:
     void reserve(size_t bytes, size_t samples, size_t frames);
     cudaStream_t stream = nullptr;
     uint8_t* d_bytes = nullptr;
-    int64_t* d_cand = nullptr;
+    struct FlacCand* d_cand = nullptr;
     FlacFrame* d_frames = nullptr;
     int* d_work = nullptr;      // frame order of the decode launch
     int16_t* d_out = nullptr;
