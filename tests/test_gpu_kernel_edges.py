@@ -123,3 +123,20 @@ def test_flac_frames_lossless(gpu, blocksize, kind):
         x = np.where(frame % 4 == 0, x, np.where(frame % 4 == 1, wave, np.where(frame % 4 == 2, 77, wave // 16)))
     x = x.astype(np.int16)
     assert np.array_equal(native.flac_decode(ldf.write(x, blocksize=blocksize, seed=blocksize)), x)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 1024, 1025, 8191, 8193, 262143, 262144, 262145])
+def test_pulse_scan_lengths(gpu, n):
+    # one warp, a ragged last word, one CTA, eight of them, and both sides of
+    # the line between one cluster and two passes; runs of NaN across words,
+    # warps and CTAs keep the state.  Integer work: identical.
+    from oracle import native as onative
+    from vhsd_gb300 import native
+    rng = np.random.default_rng(n)
+    x = rng.random(n) * 20.0 - 10.0
+    x[rng.integers(0, 20, n) == 0] = np.nan
+    for at in (n // 8 - 40, n // 2 - 700):
+        if at > 0:
+            x[at:at + 1400] = np.nan
+    for high in (0.3, -9.9, 11.0):
+        assert native.find_pulses(x, high, 1, 64) == onative.find_pulses(x, high, 1, 64)

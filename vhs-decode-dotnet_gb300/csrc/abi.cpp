@@ -1383,7 +1383,7 @@ void decode_plain(vhsdecode_gb300_session* s, const int16_t* rf_dev, uint64_t n,
         const double threshold = s->sp.ire_to_hz(s->sp.vsync_ire / 2.0);
         ck(launch_pulse_events<double>(s->s64.p, stream_len, threshold, s->pc_counts.p, s->pc_offsets.p,
                                        s->pc_events.p, s->pc_capacity, s->pc_total.p, cs), "pulse launch");
-        s->launches += kPulseKernels;
+        s->launches += (uint32_t)pulse_event_kernels(stream_len);
         int64_t total = 0;
         ck(cudaMemcpyAsync(&total, s->pc_total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, cs), "d2h");
         ck(cudaStreamSynchronize(cs), "sync");

@@ -128,7 +128,10 @@ constexpr int kPlainSubKernels = 9;     // added by sub-deemphasis (4 + 1 FFT x 
 // 1024 samples, then ordered write.  counts / offsets_scratch hold
 // pulse_count_slots(n) entries.
 constexpr int kPulseChunk = 4096;
-constexpr int kPulseKernels = 2;      // kernels one launch_pulse_events* call starts (plus a memset)
+constexpr int kPulseKernels = 2;      // kernels of a long range (plus a memset); a short range of
+                                      // samples takes one
+constexpr int64_t kPulseClusterSamples = 262144;
+inline int pulse_event_kernels(int64_t n) { return n <= 0 ? 0 : n <= kPulseClusterSamples ? 1 : kPulseKernels; }
 inline int64_t pulse_count_slots(int64_t n) { return (n + kPulseChunk - 1) / kPulseChunk * 4; }
 template <typename T>
 cudaError_t launch_pulse_events(const T* ref, int64_t n, double high, int64_t* counts,
