@@ -7,6 +7,7 @@
 // sections match the reference's to the bit wherever the C library's tan,
 // cos and sin do.
 #include "chroma.hpp"
+#include "parallel.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -285,16 +286,20 @@ void chroma_tables(const ChromaDesign& d, std::vector<float>& het, std::vector<f
     for (int p = 0; p < 4; p++) {
         const double off = (kPi / 2.0 * p) + 0.0;
         const double step = kTau * scale;
-        for (int64_t i = 0; i < n; i++) het[(size_t)(p * n + i)] = (float)(-std::cos((step * (double)i) + off));
+        parallel_ranges(n, 16384, [&](int64_t first, int64_t end) {
+            for (int64_t i = first; i < end; i++) het[(size_t)(p * n + i)] = (float)(-std::cos((step * (double)i) + off));
+        });
     }
     const double wave = d.fsc_mhz / rate;
     bsin.resize((size_t)n);
     bcos.resize((size_t)n);
-    for (int64_t i = 0; i < n; i++) {
-        float theta = (float)((kTau * wave) * (double)i);
-        bsin[(size_t)i] = numpy_trig_f32(theta, false);
-        bcos[(size_t)i] = numpy_trig_f32(theta, true);
-    }
+    parallel_ranges(n, 16384, [&](int64_t first, int64_t end) {
+        for (int64_t i = first; i < end; i++) {
+            float theta = (float)((kTau * wave) * (double)i);
+            bsin[(size_t)i] = numpy_trig_f32(theta, false);
+            bcos[(size_t)i] = numpy_trig_f32(theta, true);
+        }
+    });
 }
 
 }  // namespace vhsd

@@ -37,6 +37,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -110,11 +111,11 @@ public:
         std::unique_lock<std::mutex> lk(m_);
         cv_.wait(lk, [&] { return !q_.empty() || done_; });
         if (q_.empty()) return false;
-        std::vector<unsigned char> c = std::move(q_.front());
+        Chunk c = std::move(q_.front());
         q_.pop_front();
         lk.unlock();
         cv_.notify_all();
-        out.insert(out.end(), c.begin(), c.end());
+        out.insert(out.end(), c.p.get(), c.p.get() + c.n);
         return true;
     }
     std::string error() {
@@ -138,14 +139,14 @@ private:
                 if (off >= total) break;
                 ask = (size_t)std::min<uint64_t>(ask, total - off);
             }
-            std::vector<unsigned char> c(ask * esz_);
-            size_t got = cfg_->read_callback(cfg_->user_data, c.data(), off, ask);
+            Chunk c{std::unique_ptr<unsigned char[]>(new unsigned char[ask * esz_]), 0};   // not zeroed first
+            size_t got = cfg_->read_callback(cfg_->user_data, c.p.get(), off, ask);
             if (got > ask) {
                 std::lock_guard<std::mutex> lk(m_);
                 err_ = "read callback overran its buffer";
                 break;
             }
-            c.resize(got * esz_);
+            c.n = got * esz_;
             off += got;
             if (got) {
                 std::lock_guard<std::mutex> lk(m_);
@@ -164,7 +165,11 @@ private:
     Latch& latch_;
     std::mutex m_;
     std::condition_variable cv_;
-    std::deque<std::vector<unsigned char>> q_;
+    struct Chunk {
+        std::unique_ptr<unsigned char[]> p;
+        size_t n;
+    };
+    std::deque<Chunk> q_;
     bool stop_ = false, done_ = false;
     std::string err_;
     std::thread th_;   // last: started after the members above exist
@@ -384,6 +389,7 @@ VHSDECODE_GB300_API int32_t VHSDECODE_GB300_CALL vhsdecode_gb300_run(
         // of frames to keep the SMs busy
         Prefetch pre(config, flac_in ? 1 : esz, flac_in ? flac_read_chunk() : kReadChunk, latch);
         std::vector<unsigned char> buf;   // source samples [buf_off, buf_off + buf.size() / esz)
+        if (total) buf.reserve((size_t)(cap_src * esz));   // the first window
         uint64_t buf_off = 0;
         bool eof = false;
         FlacStreamDecoder flac;
