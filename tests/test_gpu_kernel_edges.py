@@ -140,3 +140,38 @@ def test_pulse_scan_lengths(gpu, n):
             x[at:at + 1400] = np.nan
     for high in (0.3, -9.9, 11.0):
         assert native.find_pulses(x, high, 1, 64) == onative.find_pulses(x, high, 1, 64)
+
+
+@pytest.mark.parametrize("damage", ["none", "nan_block", "nan_start", "crowded"])
+def test_pulse_edges_of_blocks(gpu, damage):
+    # the fused demodulator's edge records against the plain path's scan of its
+    # own stream: blocks without a sample (one NaN makes its whole block NaN;
+    # the first block's, and with it the state before any sample), and chunks
+    # with more edges than a record holds (a 0.4 MHz square wave around the
+    # threshold: 160 a chunk), which sends the stream through the pulse scan.
+    # Whole numbers: identical.
+    from oracle import formats
+    from vhsd_gb300 import native, synth
+    rf, _ = synth.generate(synth.config("pal_small"))
+    clean = rf.astype(np.float32)
+    x = clean.copy()
+    at = len(x) * 2 // 3
+    if damage == "nan_block":
+        x[at] = np.nan
+    elif damage == "nan_start":
+        x[5] = np.nan
+    elif damage == "crowded":
+        fmt = formats.get("PAL")["sys"]
+        t = np.arange(100000)
+        ire = np.where((t * 0.8e6 / 40e6).astype(np.int64) % 2 == 0, -60.0, 20.0)
+        x[at:at + len(t)] = 8000.0 * np.cos(2 * np.pi * np.cumsum(fmt["ire0"] + fmt["hz_ire"] * ire) / 40e6)
+    got = []
+    for precision in (native.PRECISION_FP32_FUSED, native.PRECISION_FP64_PLAIN):
+        with native.Session(native.PROFILE_PAL, len(x), precision=precision) as s:
+            r = s.decode(x)
+            got.append([(s.field(i).span_start, bool(s.field(i).is_first_field)) for i in range(r.fields)])
+            if precision == native.PRECISION_FP32_FUSED:
+                scanned = r.kernel_launches - s.decode(clean).kernel_launches
+    assert got[0] and got[0] == got[1]
+    if damage == "crowded":   # a clean decode of as many fields has no pulse scan
+        assert scanned > 0

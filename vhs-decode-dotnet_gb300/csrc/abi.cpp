@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -210,32 +211,22 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
         s->repair.alloc(1);
         s->nseg_max = (int)((std::max<int64_t>(0, s->max_blocks - kFirstSegBlocks) + kSegBlocks - 1) / kSegBlocks) + 1;
         s->seg_cap = kSegBlocks * kStride / 64 + 4096;
-        s->seg_events.alloc((size_t)s->nseg_max * s->seg_cap);
-        s->pc_counts_alt.alloc(pulse_count_slots(kSegBlocks * kStride));
-        s->pc_offsets_alt.alloc(pulse_count_slots(kSegBlocks * kStride));
-        s->seg_total.alloc((size_t)s->nseg_max);
+        s->seg_events.alloc((size_t)s->seg_cap);
         s->blk_counters.alloc((size_t)s->nseg_max + 1);   // one per segment launch, the last for run_demod
-        ck(cudaHostAlloc((void**)&s->h_events, (size_t)s->nseg_max * s->seg_cap * sizeof(int64_t),
-                         cudaHostAllocDefault), "cudaHostAlloc");
-        ck(cudaHostAlloc((void**)&s->h_totals, (size_t)s->nseg_max * sizeof(int64_t), cudaHostAllocDefault),
-           "cudaHostAlloc");
-        s->seg_done.resize((size_t)s->nseg_max);
+        const size_t edge_bytes =
+            (kEdgePad + (size_t)std::max<int64_t>(1, s->max_blocks) * kEdgeRecords * kEdgeWords) * sizeof(uint64_t);
+        ck(cudaHostAlloc((void**)&s->h_edges, edge_bytes, cudaHostAllocDefault), "cudaHostAlloc");
+        ck(cudaMemset(s->h_edges, 0, edge_bytes), "memset");   // no decode has tag 0
         s->seg_copied.resize((size_t)s->nseg_max);
-        s->seg_pulsed.resize((size_t)s->nseg_max);
         s->seg_dem.resize((size_t)s->nseg_max * 2);
-        s->seg_demod_end.resize((size_t)s->nseg_max);
-        for (auto& e : s->seg_demod_end) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-        for (auto& e : s->seg_done) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         for (auto& e : s->seg_copied) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-        for (auto& e : s->seg_pulsed) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         for (auto& e : s->seg_dem) ck(cudaEventCreate(&e), "cudaEventCreate");
         ck(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
-        ck(cudaStreamCreateWithFlags(&s->d2h_stream, cudaStreamNonBlocking), "cudaStreamCreate");
         ck(cudaStreamCreateWithFlags(&s->alt_stream, cudaStreamNonBlocking), "cudaStreamCreate");
         ck(cudaEventCreateWithFlags(&s->alt_start, cudaEventDisableTiming), "cudaEventCreate");
         ck(cudaEventCreateWithFlags(&s->alt_end, cudaEventDisableTiming), "cudaEventCreate");
         ck(cudaEventCreateWithFlags(&s->copy_end, cudaEventDisableTiming), "cudaEventCreate");
-        ck(cudaEventCreateWithFlags(&s->d2h_end, cudaEventDisableTiming), "cudaEventCreate");
+        ck(cudaEventCreateWithFlags(&s->pipe_end, cudaEventDisableTiming), "cudaEventCreate");
         ck(cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking), "cudaStreamCreate");
         s->fft_plan = tuned_fft_plan(s, fp32_params(s, nullptr));
     } else {
@@ -506,19 +497,17 @@ void session_free(vhsdecode_gb300_session* s) {
     if (s->chroma_stream) cudaStreamDestroy(s->chroma_stream);
     if (s->demod_cycles) cudaFree(s->demod_cycles);
     for (auto& ev : s->ev) if (ev) cudaEventDestroy(ev);
-    for (auto* v : {&s->seg_done, &s->seg_copied, &s->seg_pulsed, &s->seg_dem, &s->seg_demod_end})
+    for (auto* v : {&s->seg_copied, &s->seg_dem})
         for (auto& ev : *v) if (ev) cudaEventDestroy(ev);
-    if (s->h_events) cudaFreeHost(s->h_events);
+    if (s->h_edges) cudaFreeHost(s->h_edges);
     if (s->h_field_in) cudaFreeHost(s->h_field_in);
     if (s->h_field_out) cudaFreeHost(s->h_field_out);
-    if (s->h_totals) cudaFreeHost(s->h_totals);
     if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
-    if (s->d2h_stream) cudaStreamDestroy(s->d2h_stream);
     if (s->alt_stream) cudaStreamDestroy(s->alt_stream);
     if (s->alt_start) cudaEventDestroy(s->alt_start);
     if (s->alt_end) cudaEventDestroy(s->alt_end);
     if (s->copy_end) cudaEventDestroy(s->copy_end);
-    if (s->d2h_end) cudaEventDestroy(s->d2h_end);
+    if (s->pipe_end) cudaEventDestroy(s->pipe_end);
     if (s->pipe_exec) cudaGraphExecDestroy(s->pipe_exec);
     if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
     if (s->aux_stream) cudaStreamDestroy(s->aux_stream);
@@ -630,7 +619,8 @@ int tuned_fft_plan(vhsdecode_gb300_session* s, FastDemodParams base) {
 
 // The fused demodulator, or (VHSD_DEMOD_TIMING set) its timed diagnostic build.
 cudaError_t launch_fused(vhsdecode_gb300_session* s, FastDemodParams p, cudaStream_t st) {
-    const int clusters = s->demod_clusters > 0 ? s->demod_clusters : s->num_sms / 2;
+    const int clusters =
+        s->demod_clusters > 0 && p.first_claims == INT_MAX ? s->demod_clusters : s->num_sms / 2;
     if (!s->demod_cycles) return launch_demod_fp32(p, clusters, st);
     p.stage_cycles = s->demod_cycles;
     return launch_demod_fp32_timed(p, clusters, st);
@@ -669,6 +659,7 @@ FastDemodParams fp32_params(vhsdecode_gb300_session* s, const int16_t* rf_dev) {
     p.rf_f32 = s->in_f32;
     if (s->in_f32) p.rf = nullptr;
     p.block_counter = nullptr;
+    p.first_claims = INT_MAX;
     p.sync_cond = s->sync_cond.p;
     p.sync_hold = s->sync_hold.p;
     p.sync_thr = pulse_float_threshold(s->sp.ire_to_hz(s->sp.vsync_ire / 2.0));
@@ -731,7 +722,8 @@ struct EventFeed {
 // TbcFieldSequenceDecodeEngine order (Core/Decode/TbcFieldSequenceDecodeEngine.cs:442-560):
 // resolve the next field span, take its pulses, run the control plane, step by
 // the next-field offset.  The long-hsync rescue reads the sync reference of a
-// finished span on the auxiliary stream, so it never waits behind queued work.
+// finished span on the auxiliary stream, so it waits for the demodulation but
+// for no other queued work.
 template <typename T>
 void host_field_loop(vhsdecode_gb300_session* s, const T* sync, int64_t stream_len, uint32_t max_fields,
                      EventFeed& feed, uint32_t& stop_reason, const std::atomic<bool>* cancel,
@@ -760,6 +752,8 @@ void host_field_loop(vhsdecode_gb300_session* s, const T* sync, int64_t stream_l
                                              min_len, max_len);
         RefFetch fetch = [&](int64_t start, int64_t len, std::vector<double>& out) {
             tmp.resize((size_t)len);
+            // an edge record says nothing about the sync samples of its block
+            if (s->edges_pending) ck(cudaStreamWaitEvent(s->aux_stream, s->pipe_end, 0), "rescue fetch");
             ck(cudaMemcpyAsync(tmp.data(), sync + s0 + start, (size_t)len * sizeof(T),
                                cudaMemcpyDeviceToHost, s->aux_stream), "rescue fetch");
             ck(cudaStreamSynchronize(s->aux_stream), "rescue fetch");
@@ -1133,7 +1127,7 @@ void collect_field_results(vhsdecode_gb300_session* s, cudaStream_t fs) {
 }
 
 // Segment boundaries (in blocks) of the pipelined decode: a short first
-// segment so the control plane can start early, then kSegBlocks each.
+// segment so the demod can start soon behind its RF copy, then kSegBlocks each.
 std::vector<int64_t> segment_bounds(int64_t nblocks) {
     std::vector<int64_t> b{0};
     int64_t e = std::min<int64_t>(nblocks, kFirstSegBlocks);
@@ -1144,18 +1138,10 @@ std::vector<int64_t> segment_bounds(int64_t nblocks) {
     return b;
 }
 
-// FP32 decode, pipelined: the capture is demodulated in segments; after each
-// segment the device writes that segment's pulse events and copies them to
-// pinned host memory, so the host control plane analyses the fields of
-// finished segments while later segments are still being demodulated.  With
-// host input the RF of each segment is copied on a separate stream ahead of
-// its demod.  Results are identical to a single pass: demod blocks are
-// independent and the ranged pulse scan carries its state across segments.
-// Queues the segment pipeline from `root`: RF copies on copy_stream, demod and
-// pulse scans alternating between root and alt_stream, event copies on
-// d2h_stream; every side stream joins back into root at the end.  When
-// `capturing`, the events the host waits on or times (seg_done, seg_dem) are
-// recorded as external graph nodes.
+// Queues the demodulator's segments from `root`: RF copies on copy_stream,
+// launches alternating between root and alt_stream; both join back into root
+// at the end.  When `capturing`, the events the host waits on or times
+// (seg_dem) are recorded as external graph nodes.
 void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n, bool host_input,
                       bool demod_only, const std::vector<int64_t>& bounds, cudaStream_t root, bool capturing) {
     auto rec = [&](cudaEvent_t e, cudaStream_t st, bool external) {
@@ -1165,11 +1151,15 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
     const int nseg = (int)bounds.size() - 1;
     const int16_t* rf_dev = host_input ? s->rf.p : rf;
     FastDemodParams p = fp32_params(s, rf_dev);
+    if (!demod_only) {
+        p.edges = reinterpret_cast<unsigned long long*>(s->h_edges + kEdgePad);
+        p.edge_tag_at = reinterpret_cast<const unsigned*>(s->h_edges);
+    }
     ck(cudaMemsetAsync(s->repair.p, 0, sizeof(int), root), "memset");
+    ck(cudaMemsetAsync(s->blk_counters.p, 0, (size_t)nseg * sizeof(unsigned), root), "memset");
     rec(s->alt_start, root, false);
     ck(cudaStreamWaitEvent(s->alt_stream, s->alt_start, 0), "wait");
     ck(cudaStreamWaitEvent(s->copy_stream, s->alt_start, 0), "wait");
-    ck(cudaStreamWaitEvent(s->d2h_stream, s->alt_start, 0), "wait");
     int64_t copied = 0;
     for (int k = 0; k < nseg; k++) {
         int64_t b0 = bounds[(size_t)k], b1 = bounds[(size_t)k + 1];
@@ -1189,50 +1179,111 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
         const size_t half = (size_t)(s->num_sms / 2) * kBlock;
         p.scratch = s->scratch.p + (k & 1) * 2 * half;
         p.block_counter = s->blk_counters.p + k;
-        ck(cudaMemsetAsync(p.block_counter, 0, sizeof(unsigned), ks), "memset");
+        // one launch beside the chroma block stage: clusters for its SMs too, once they are free
+        p.first_claims = !host_input && s->demod_clusters > 0 ? s->demod_clusters : INT_MAX;
         rec(s->seg_dem[(size_t)(2 * k)], ks, true);
         ck(launch_fused(s, p, ks), "demod fp32 launch");
         rec(s->seg_dem[(size_t)(2 * k + 1)], ks, true);
-        rec(s->seg_demod_end[(size_t)k], ks, false);   // dependency edge (the timing record above is external)
-        if (!demod_only) {
-            // the scan needs the previous segment's samples (state before b0)
-            if (k > 0) ck(cudaStreamWaitEvent(ks, s->seg_demod_end[(size_t)k - 1], 0), "wait");
-            int64_t* ev = s->seg_events.p + (size_t)k * s->seg_cap;
-            int64_t* cnt = (k & 1) ? s->pc_counts_alt.p : s->pc_counts.p;
-            int64_t* off = (k & 1) ? s->pc_offsets_alt.p : s->pc_offsets.p;
-            // from the pulse-scan bits the demod wrote with the sync stream
-            ck(launch_pulse_bits_range(s->sync_cond.p, s->sync_hold.p, b0 * kStride, b1 * kStride, cnt, off, ev,
-                                       s->seg_cap, s->seg_total.p + k, ks), "pulse launch");
-            rec(s->seg_pulsed[(size_t)k], ks, false);
-            ck(cudaStreamWaitEvent(s->d2h_stream, s->seg_pulsed[(size_t)k], 0), "wait");
-            ck(cudaMemcpyAsync(s->h_totals + k, s->seg_total.p + k, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                               s->d2h_stream), "d2h");
-            ck(cudaMemcpyAsync(s->h_events + (size_t)k * s->seg_cap, ev, (size_t)s->seg_cap * sizeof(int64_t),
-                               cudaMemcpyDeviceToHost, s->d2h_stream), "d2h events");
-            rec(s->seg_done[(size_t)k], s->d2h_stream, true);
-        }
     }
     // join the side streams back into root
-    for (cudaStream_t side : {s->alt_stream, s->copy_stream, s->d2h_stream}) {
-        cudaEvent_t j = side == s->alt_stream ? s->alt_end : (side == s->copy_stream ? s->copy_end : s->d2h_end);
+    for (cudaStream_t side : {s->alt_stream, s->copy_stream}) {
+        cudaEvent_t j = side == s->alt_stream ? s->alt_end : s->copy_end;
         rec(j, side, false);
         ck(cudaStreamWaitEvent(root, j, 0), "wait");
     }
 }
 
-// Kernels the pipeline queues for `bounds` (demod + pulse scans).
-uint32_t pipeline_launches(const std::vector<int64_t>& bounds, bool demod_only) {
-    uint32_t nseg = (uint32_t)(bounds.size() - 1);
-    return nseg * (1u + (demod_only ? 0u : (uint32_t)kPulseKernels));
-}
+// Pulse events of the stitched stream as the demodulator finishes its blocks:
+// the blocks' edge records (FastDemodParams::edges) are taken in stream order,
+// each joined to the state that the one before ends in.  A record with more
+// edges than it holds sends the whole stream through the pulse scan instead,
+// once the demodulation queued on `cs` is over.
+class EdgeReader {
+public:
+    EdgeReader(vhsdecode_gb300_session* s, int64_t nblocks, cudaStream_t cs)
+        : s_(s), nblocks_(nblocks), cs_(cs) {}
+    void upto(int64_t pos, std::vector<int64_t>& events) {
+        while (next_ * kStride < pos && next_ < nblocks_) {
+            if (!take_block(events)) {
+                scan_stream(events);
+                next_ = nblocks_;
+                return;
+            }
+            next_++;
+        }
+    }
 
-// FP32 decode, pipelined: the capture is demodulated in segments; after each
-// segment the device writes that segment's pulse events and copies them to
-// pinned host memory, so the host control plane analyses the fields of
-// finished segments while later segments are still being demodulated.  With
-// host input the RF of each segment is copied on a separate stream ahead of
-// its demod.  Results are identical to a single pass: demod blocks are
-// independent and the ranged pulse scan carries its state across segments.
+private:
+    // The word at `w` once it is of this decode.  The demodulator's end is
+    // looked at now and then, so that its failure ends the wait.
+    uint64_t wait_word(const uint64_t* w) {
+        for (unsigned spin = 1;; spin++) {
+            uint64_t v = __atomic_load_n(w, __ATOMIC_ACQUIRE);
+            if ((uint32_t)(v >> 32) == s_->edge_tag) return v;
+            if (spin & 1023u) continue;
+            const cudaError_t q = cudaEventQuery(s_->pipe_end);
+            if (q == cudaErrorNotReady) {
+                cudaGetLastError();
+                continue;
+            }
+            ck(q, "segment wait");
+            v = __atomic_load_n(w, __ATOMIC_ACQUIRE);
+            if ((uint32_t)(v >> 32) == s_->edge_tag) return v;
+            throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "a block's pulse edges are missing");
+        }
+    }
+    bool take_block(std::vector<int64_t>& events) {
+        const uint64_t* rec = s_->h_edges + kEdgePad + (size_t)next_ * kEdgeRecords * kEdgeWords;
+        const int64_t base = 2 * next_ * kStride;
+        for (int c = 0; c < kEdgeRecords; c++, rec += kEdgeWords) {
+            // two blocks on: the records lie a kilobyte apart
+            if (next_ + 2 < nblocks_) __builtin_prefetch(rec + 2 * kEdgeRecords * kEdgeWords);
+            const uint32_t h = (uint32_t)wait_word(rec);
+            const int count = (int)(h & 16383u);
+            if (count > kEdgeCap) return false;
+            if (!((h >> 29) & 1u)) continue;
+            const bool first = (h >> 27) & 1u;
+            if (first != state_)
+                events.push_back(base + 2 * (c * (kBlock / 4) + (int64_t)((h >> 14) & 8191u) - kCut - 32) + (first ? 0 : 1));
+            for (int i = 1; i <= count; i++) events.push_back(base + (int64_t)(uint32_t)wait_word(rec + i));
+            state_ = (h >> 28) & 1u;
+        }
+        return true;
+    }
+    void scan_stream(std::vector<int64_t>& events) {
+        ck(cudaStreamSynchronize(cs_), "segment wait");
+        events.clear();
+        const std::vector<int64_t> bounds = segment_bounds(nblocks_);
+        for (size_t k = 0; k + 1 < bounds.size(); k++) {
+            ck(launch_pulse_bits_range(s_->sync_cond.p, s_->sync_hold.p, bounds[k] * kStride, bounds[k + 1] * kStride,
+                                       s_->pc_counts.p, s_->pc_offsets.p, s_->seg_events.p, s_->seg_cap,
+                                       s_->pc_total.p, cs_), "pulse launch");
+            s_->launches += kPulseKernels;
+            int64_t total = 0;
+            ck(cudaMemcpyAsync(&total, s_->pc_total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, cs_), "d2h");
+            ck(cudaStreamSynchronize(cs_), "sync");
+            if (total > s_->seg_cap)
+                throw Failure(VHSDECODE_GB300_STATUS_DECODE_ERROR, "sync pulse event capacity exceeded");
+            const size_t at = events.size();
+            events.resize(at + (size_t)total);
+            if (total)
+                ck(cudaMemcpy(events.data() + at, s_->seg_events.p, (size_t)total * sizeof(int64_t),
+                              cudaMemcpyDeviceToHost), "d2h events");
+        }
+    }
+    vhsdecode_gb300_session* s_;
+    int64_t nblocks_, next_ = 0;
+    cudaStream_t cs_;
+    bool state_ = false;
+};
+
+// FP32 decode, pipelined: the demodulator writes each block's pulse edges to
+// pinned host memory as it goes, so the host control plane analyses the fields
+// of finished blocks while later ones are still being demodulated.  A capture
+// on the device is demodulated by one launch; one in host memory in segments,
+// the RF of each copied on a separate stream ahead of its launch.  Results are
+// identical to a single pass: blocks are independent, and the host carries the
+// state of the pulse scan from block to block.
 // With device input or pinned host input the queued work is captured once as
 // a CUDA graph (keyed by the input pointer, length and mode) and replayed.
 void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n, bool host_input,
@@ -1241,12 +1292,6 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     cudaStream_t cs = s->stream;
     int64_t nblocks = block_count(n);
     int64_t stream_len = nblocks * kStride;
-    // with no field work to overlap, the demod runs as one launch
-    std::vector<int64_t> bounds = demod_only ? std::vector<int64_t>{0, nblocks} : segment_bounds(nblocks);
-    if (nblocks == 0) bounds.assign(1, 0);
-    int nseg = (int)bounds.size() - 1;
-    s->segments = (uint32_t)nseg;
-    if (nseg > s->nseg_max) throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "segment table too small");
     auto tq0 = std::chrono::steady_clock::now();
     bool graphable = !host_input;
     if (host_input && n > 0) {
@@ -1291,6 +1336,22 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         ck(cudaEventRecord(s->chroma_go, cs), "event");
         queue_chroma_blocks(s, rf, nblocks, s->chroma_go);
     }
+    // with nothing to overlap (copies), the demod runs as one launch
+    std::vector<int64_t> bounds = demod_only || !host_input ? std::vector<int64_t>{0, nblocks} : segment_bounds(nblocks);
+    if (nblocks == 0) bounds.assign(1, 0);
+    const int nseg = (int)bounds.size() - 1;
+    s->segments = (uint32_t)nseg;
+    if (nseg > s->nseg_max) throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "segment table too small");
+    if (!demod_only && nseg > 0) {
+        // a demod that an earlier decode left behind (it failed) reads the tag when it starts
+        if (s->edges_pending) ck(cudaStreamSynchronize(cs), "sync");
+        if (++s->edge_tag == 0) {   // 2^32 decodes on: no word may look new
+            std::memset(s->h_edges, 0, (kEdgePad + (size_t)s->max_blocks * kEdgeRecords * kEdgeWords) * sizeof(uint64_t));
+            s->edge_tag = 1;
+        }
+        __atomic_store_n(reinterpret_cast<uint32_t*>(s->h_edges), s->edge_tag, __ATOMIC_RELEASE);
+        s->edges_pending = true;
+    }
     if (graphable && nseg > 0) {
         PipeKey key{s->in_f32 ? (const void*)s->in_f32 : (const void*)rf, n, host_input, demod_only,
                     s->in_f32 != nullptr, s->demod_clusters};
@@ -1318,25 +1379,14 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     } else {
         enqueue_pipeline(s, rf, n, host_input, demod_only, bounds, cs, false);
     }
-    s->launches += pipeline_launches(bounds, demod_only);
+    ck(cudaEventRecord(s->pipe_end, cs), "event");
+    s->launches += (uint32_t)nseg;
     s->enqueue_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tq0).count();
     if (!demod_only && nblocks > 0) {
         auto t0 = std::chrono::steady_clock::now();
         EventFeed feed;
-        int kdone = 0;
-        int64_t ready = 0;
-        feed.upto = [&](int64_t pos) {
-            while (ready < pos && kdone < nseg) {
-                ck(cudaEventSynchronize(s->seg_done[(size_t)kdone]), "segment wait");
-                int64_t cnt = s->h_totals[kdone];
-                if (cnt > s->seg_cap)
-                    throw Failure(VHSDECODE_GB300_STATUS_DECODE_ERROR, "sync pulse event capacity exceeded");
-                const int64_t* e = s->h_events + (size_t)kdone * s->seg_cap;
-                feed.events.insert(feed.events.end(), e, e + cnt);
-                ready = bounds[(size_t)kdone + 1] * kStride;
-                kdone++;
-            }
-        };
+        EdgeReader edges(s, nblocks, cs);
+        feed.upto = [&](int64_t pos) { edges.upto(pos, feed.events); };
         // The field kernels run as one batch over all fields after the host
         // loop: batches launched from the host loop while the closing segments
         // demodulate were slower (host launch and copy time lands on the
@@ -1344,6 +1394,8 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         host_field_loop<float>(s, s->s32.p, stream_len, max_fields, feed, stop, cancel, carry);
         host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         ck(cudaEventRecord(s->ev[2], cs), "event");
+        // (the host saw the pulse edges of the fields' blocks, not their streams)
+        ck(cudaStreamWaitEvent(s->field_stream, s->ev[2], 0), "wait");
         launch_field_batch<float>(s, 0, (int)s->fields.size(), s->v32.p, s->s32.p, s->e32.p,
                                   stream_len, s->field_stream);
         collect_field_results(s, s->field_stream);
@@ -1353,8 +1405,8 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         ck(cudaEventRecord(s->ev[2], cs), "event");
     }
     finish_chroma_blocks(s, cs);
-    ck(cudaStreamSynchronize(s->d2h_stream), "sync");
     ck(cudaEventSynchronize(s->seg_dem[(size_t)(2 * std::max(0, nseg - 1) + 1)]), "sync");
+    s->edges_pending = false;
     demod_ms = 0.0f;
     for (int k = 0; k < nseg; k++) {
         float t = 0.0f;

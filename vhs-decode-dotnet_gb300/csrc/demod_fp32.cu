@@ -43,6 +43,7 @@
 #include <stdint.h>
 
 #include "fft_common.cuh"
+#include "pulse_bits.cuh"
 #include "spikes.cuh"
 #include "vhs_math.cuh"
 #include "kernels.h"
@@ -185,14 +186,16 @@ __device__ __forceinline__ void fft16384(float2* buf, const Tw& tw, int tid) {
 struct Shared {
     float2 buf[BUF];
     float theta[M];          // stage 3: angle, then demod, of each local sample
-    unsigned repl[N / 32];   // spike windows chosen for replacement (repair path)
+    unsigned repl[N / 32];   // spike windows chosen for replacement (repair path), later
+                             // the rank's pulse-scan words: condition, then hold
     Tw tw;
     float2 nyq;              // Nyquist bin of the rank-0 half spectrum
     float2 tail_z[2][2];     // last two analytic samples of each local chunk
     float tail_theta[2];     // last angle of each local chunk
     float tail_re[2][4];     // last four Re z of each local chunk
     int flag;
-    int pad_;
+    unsigned edge_tag;       // the decode's tag of the pulse edges
+    unsigned edge_sum[T / 32];   // each warp's edges, and its first and last state
     long long next_blk[2];   // the cluster's next block, by iteration parity
     int next_job[2];         // batched launch: the next block's window
     int cur_job;
@@ -569,8 +572,9 @@ __device__ __forceinline__ unsigned spread16(unsigned x) {
 // 2 lane + 1 (q.x, q.y) held by the 32 lanes of a warp: condition (v <= the
 // exact float threshold of the pulse scan) and hold (NaN) words for stream
 // samples [sbase + base, sbase + base + 64), written where the word lies in
-// the kept range.  Called by all 32 lanes.
-__device__ __forceinline__ void sync_bits(float2 q, int base, int64_t sbase, const FastDemodParams& p,
+// the kept range, to the stream's words and the rank's own (sh.repl).  Called
+// by all 32 lanes.
+__device__ __forceinline__ void sync_bits(Shared& sh, float2 q, int base, int64_t sbase, const FastDemodParams& p,
                                           int lane) {
     const unsigned ce = __ballot_sync(0xffffffffu, q.x <= p.sync_thr);
     const unsigned co = __ballot_sync(0xffffffffu, q.y <= p.sync_thr);
@@ -579,14 +583,97 @@ __device__ __forceinline__ void sync_bits(float2 q, int base, int64_t sbase, con
     if (lane < 2) {
         const int n = base + 32 * lane;   // first block sample of this lane's word
         if (n >= CUT + 32 && n + 32 <= CUT + 32 + S) {
-            const int sh = 16 * lane;
-            const unsigned c = spread16(ce >> sh) | (spread16(co >> sh) << 1);
-            const unsigned h = spread16(he >> sh) | (spread16(ho >> sh) << 1);
+            const int half = 16 * lane;
+            const unsigned c = spread16(ce >> half) | (spread16(co >> half) << 1);
+            const unsigned h = spread16(he >> half) | (spread16(ho >> half) << 1);
             const int64_t w = (sbase + n) >> 5;
             p.sync_cond[w] = c;
             p.sync_hold[w] = h;
+            const int slot = ((n >> 14) << 8) | ((n & 8191) >> 5);
+            sh.repl[slot] = c;
+            sh.repl[T + slot] = h;
         }
     }
+}
+
+// Pulse edges of this rank's two chunks (FastDemodParams::edges) from the
+// words of sync_bits, a word a thread.  The host reads them while later blocks
+// are being demodulated.  Two scan kernels behind each segment of blocks did
+// this before: a demod CTA fills its SM, so the scans waited for CTAs of the
+// next segment to run dry, and the segment after that waited for the scans (60
+// NTSC fields, luma, from pinned memory: last event at 1.45 ms, 1.41 now, of
+// which the records cost 3,800 of a block's 150,000 cycles).  The words carry
+// the tag instead of a fence ahead of the header: a fence to the system's scope
+// cost another 5,000 cycles a block, one to the device's 2,000.  Called by
+// every thread, after a barrier behind sync_bits.
+__device__ __noinline__ void write_edges(Shared& sh, const FastDemodParams& p, unsigned tag32, int64_t blk,
+                                         int rank) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c = 2 * (tid >> 8) + rank;
+    const int n = c * 8192 + 32 * (tid & 255);
+    const bool kept = n >= CUT + 32 && n < CUT + 32 + S;
+    const unsigned cw = kept ? sh.repl[tid] : 0u;
+    const unsigned hw = kept ? sh.repl[T + tid] : 0xffffffffu;
+    const bool has = hw != 0xffffffffu;
+    const int b_first = has ? __ffs(~hw) - 1 : 0;
+    const unsigned first = has ? (cw >> b_first) & 1u : 0u;
+    const unsigned last = has ? (cw >> (31 - __clz(~hw))) & 1u : 0u;
+    const unsigned hm = __ballot_sync(0xffffffffu, has);
+    const unsigned before = hm & ((1u << lane) - 1u);
+    const unsigned from = __shfl_sync(0xffffffffu, last, before ? 31 - __clz(before) : 0);
+    // edges inside the warp's 1024 samples: no state is known before its first one
+    unsigned st = before ? from : first;
+    unsigned e = edge_bits(cw, hw, st);
+    const int pc = __popc(e);
+    int incl = pc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const int head = hm ? __ffs(hm) - 1 : 0;
+    {
+        const unsigned w_first = __shfl_sync(0xffffffffu, first, head);
+        const unsigned w_last = __shfl_sync(0xffffffffu, last, hm ? 31 - __clz(hm) : 0);
+        const unsigned w_at = 32 * head + __shfl_sync(0xffffffffu, b_first, head);
+        const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 0)
+            sh.edge_sum[warp] = total | (w_at << 11) | (w_first << 21) | (w_last << 22) | ((hm ? 1u : 0u) << 23);
+    }
+    __syncthreads();
+    // the chunk's eight warps joined: an edge where a warp starts in another state than the one before ends
+    unsigned known = 0, state = 0, count = 0, off = 0, extra = 0, first_state = 0, first_at = 0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+        const unsigned s = sh.edge_sum[(warp & 8) + v];
+        if (v == (warp & 7)) off = count;
+        if (!(s >> 23)) continue;
+        const unsigned x = known & (((s >> 21) & 1u) ^ state);
+        if (v == (warp & 7)) extra = x;
+        if (!known) {
+            first_state = (s >> 21) & 1u;
+            first_at = 1024 * v + ((s >> 11) & 1023u);
+        }
+        count += (s & 2047u) + x;
+        state = (s >> 22) & 1u;
+        known = 1;
+    }
+    if (extra && lane == head) e |= 1u << b_first;
+    unsigned o = off + (unsigned)(incl - pc) + (extra && lane > head ? 1u : 0u);
+    const unsigned long long tag = (unsigned long long)tag32 << 32;
+    unsigned long long* rec = p.edges + ((blk + p.first_block) * kEdgeRecords + c) * (int64_t)kEdgeWords;
+    auto store = [](unsigned long long* at, unsigned long long v) {
+        asm volatile("st.relaxed.sys.global.u64 [%0], %1;\n" ::"l"(at), "l"(v) : "memory");
+    };
+    while (e) {
+        const int b = __ffs(e) - 1;
+        e &= e - 1;
+        if (o < (unsigned)kEdgeCap)
+            store(rec + 1 + o, tag | (unsigned)(2 * (n + b - CUT - 32) + (((cw >> b) & 1u) ? 0 : 1)));
+        o++;
+    }
+    if ((tid & 255) == 0)
+        store(rec, tag | count | (first_at << 14) | (first_state << 27) | (state << 28) | (known << 29));
 }
 
 // Next block's RF (32768 int16 = 64 KB, both halves) into `dst` with
@@ -663,6 +750,10 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
     Shared* rsh = cluster.map_shared_rank(&sh, rank ^ 1);
     float2* rbuf = rsh->buf;
 
+    const int cluster_id = blockIdx.x >> 1;
+    const int nclusters = gridDim.x >> 1;
+    // clusters that start on their own block
+    const int nstatic = BATCHED ? nclusters : min(nclusters, pk.first_claims);
     for (int i = tid; i < 256; i += T) sh.tw.hi[i] = pk.tw_hi[i];
     for (int i = tid; i < 128; i += T) sh.tw.lo[i] = pk.tw_lo[i];
     for (int i = tid; i < 16; i += T) sh.tw.lo8[i] = pk.tw_lo[8 * i];
@@ -671,8 +762,17 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
     }
     __syncthreads();
 
-    const int cluster_id = blockIdx.x >> 1;
-    const int nclusters = gridDim.x >> 1;
+    int64_t g0 = cluster_id;
+    if (cluster_id >= nstatic) {
+        cluster.sync();
+        if (rank == 0 && tid == 0) {
+            const long long nb = (long long)nstatic + atomicAdd(pk.block_counter, 1);
+            sh.next_blk[1] = nb;
+            rsh->next_blk[1] = nb;
+        }
+        cluster.sync();
+        g0 = sh.next_blk[1];
+    }
     const float inv_n = 1.0f / (float)N;
     const float inv_m = 1.0f / (float)M;
     // the RF of each block is prefetched into sh.theta (free from the demod's
@@ -682,24 +782,29 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
     // (batched launches take int16 captures only)
     const int16_t* rf_smem = reinterpret_cast<const int16_t*>(sh.theta);
     const bool f32_in = !BATCHED && pk.rf_f32 != nullptr;
-    if (cluster_id < pk.nblocks && !f32_in) {
+    if (g0 < pk.nblocks && !f32_in) {
         if constexpr (BATCHED) {
             const FastDemodParams& j0 = pk.batch_jobs[sh.cur_job];
             prefetch_rf(sh.theta, j0.rf + (cluster_id - pk.batch_start[sh.cur_job] + j0.first_block) * (int64_t)S,
                         tid);
         } else {
-            prefetch_rf(sh.theta, pk.rf + (cluster_id + pk.first_block) * (int64_t)S, tid);
+            prefetch_rf(sh.theta, pk.rf + (g0 + pk.first_block) * (int64_t)S, tid);
         }
     }
-    // Blocks: each cluster starts on block cluster_id and then claims the next
+    if constexpr (!BATCHED) {
+        if (tid == 0 && pk.edges)
+            sh.edge_tag = pk.edge_tag_at ? *reinterpret_cast<const volatile unsigned*>(pk.edge_tag_at) : pk.edge_tag;
+    }
+    // Blocks: each cluster starts on block cluster_id (those that may start
+    // late, from first_claims on, claim that one too) and then claims the next
     // unclaimed block from the launch's counter, so clusters that start late
     // (their SMs busy with other work) or take the slow repair path simply
-    // take fewer blocks.  Rank 0 claims at the top of a block and publishes the
+    // take fewer blocks, and blocks finish in about their order.  Rank 0 claims at the top of a block and publishes the
     // index to both CTAs (slot by iteration parity); both read it after the
     // next cluster barrier, so the two ranks always agree.
     int par = 0;
     int job = -1;
-    for (int64_t g = cluster_id; g < pk.nblocks;) {
+    for (int64_t g = g0; g < pk.nblocks;) {
         // g: the block's index in the launch; blk: its index in its window
         int64_t blk = g;
         if constexpr (BATCHED) {
@@ -716,7 +821,7 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         const FastDemodParams& p = BATCHED ? sh.job : pk;
         const float freq = p.fs;
         if (rank == 0 && tid == 0) {
-            const long long nb = pk.block_counter ? (long long)nclusters + atomicAdd(pk.block_counter, 1)
+            const long long nb = pk.block_counter ? (long long)nstatic + atomicAdd(pk.block_counter, 1)
                                                   : (long long)(g + nclusters);
             sh.next_blk[par] = nb;
             rsh->next_blk[par] = nb;
@@ -1000,12 +1105,16 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
                             // NaN, for the warp's 64 consecutive samples of each half
                             const int64_t sbase = (blk + p.first_block) * (int64_t)S - CUT - 32;
                             const int base1 = 2 * (m - lane);
-                            sync_bits(q1, base1, sbase, p, lane);
-                            sync_bits(q2, base1 + 16384, sbase, p, lane);
+                            sync_bits(sh, q1, base1, sbase, p, lane);
+                            sync_bits(sh, q2, base1 + 16384, sbase, p, lane);
                         }
                     }
                 }
             }
+        }
+        if (p.edges) {
+            __syncthreads();
+            write_edges(sh, p, BATCHED ? p.edge_tag : sh.edge_tag, blk, rank);
         }
         VHSD_MARK(17);
         if (sub) {

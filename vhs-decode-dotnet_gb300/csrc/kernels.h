@@ -32,6 +32,8 @@ struct FastDemodParams {
     const int16_t* rf;         // capture, 16-byte aligned
     const float* rf_f32;       // float capture (16-byte aligned), read instead of rf when set
     unsigned* block_counter;   // zeroed before the launch: dynamic block claims (null: static schedule)
+    int first_claims;          // clusters from this one on claim their first block too (with block_counter;
+                               // launched for SMs that other work holds at the start)
     int64_t first_block;       // first 32768-sample block to decode
     int64_t nblocks;           // number of blocks
     const float* rf_video;     // [kHalf] real RF band-pass gain
@@ -56,6 +58,18 @@ struct FastDemodParams {
     unsigned* sync_cond;
     unsigned* sync_hold;
     float sync_thr;
+    // optional pulse edges of each block, in pinned host memory (null: not
+    // written): per stream block four records of kEdgeWords words, one for each
+    // 8192-sample chunk.  A word's upper half is the decode's tag, *edge_tag_at
+    // (or edge_tag where that is null), so the host tells a word of this
+    // decode from an older one.  Word 0, written last, is the chunk's header
+    // (edge_header below); words 1.. hold its edges in stream order: 2 x the
+    // position in the block's 30720 stream samples, + 1 where the signal rises
+    // through sync_thr.  The chunk's first non-NaN sample makes no edge here:
+    // the state before it is the previous chunk's, which the host knows.
+    unsigned long long* edges;
+    const unsigned* edge_tag_at;
+    unsigned edge_tag;
     // diagnostics only (launch_demod_fp32_timed): per-rank cycle sums of the
     // kernel's stages, [rank * kDemodStages + stage]
     unsigned long long* stage_cycles;
@@ -68,6 +82,16 @@ struct FastDemodParams {
     int batch_njobs;
 };
 constexpr int kDemodStages = 20;
+// Edge records: a header and up to kEdgeCap edges.  A chunk holds about three
+// lines (seven edges; fourteen in a vertical interval), the 0.5 MHz sync
+// filter passes at most about a hundred crossings a chunk; a chunk with more
+// is left to the pulse scan of the whole stream.  The lower half of a header:
+// bits 0-13 the chunk's edges, 14-26 its first non-NaN sample, 27 and 28 the
+// states of its first and last one (1: v <= threshold), 29 whether it has any.
+constexpr int kEdgeWords = 128;
+constexpr int kEdgeCap = kEdgeWords - 1;
+constexpr int kEdgeRecords = 4;   // per block
+constexpr int kEdgePad = 16;      // words ahead of the records: the first holds the decode's tag
 // Radix plans the fused kernel is compiled for (8192-point plan | 16384-point
 // plan << 2): 16x16x32 | 16x32x32, 32x16x16 | 16x32x32, 16x16x32 | 32x32x16,
 // 32x16x16 | 32x32x16.  The other plans of the transforms (16x32x16, 8x32x32;

@@ -165,7 +165,6 @@ struct vhsdecode_gb300_session {
     DevBuf<unsigned> pmask;
     DevBuf<double2> ptwiddle;
     DevBuf<int64_t> pc_counts, pc_offsets, pc_events, pc_total;
-    DevBuf<int64_t> pc_counts_alt, pc_offsets_alt;   // scan scratch of odd segments
     int64_t pc_capacity = 0;
     // the field stage's per-field inputs, carved from one device block that is
     // filled from its pinned host mirror (same layout) by one copy per decode
@@ -182,24 +181,25 @@ struct vhsdecode_gb300_session {
     // counts and status, and the first kDropEarly dropout triplets of each field
     unsigned char* h_field_out = nullptr;
     DevBuf<unsigned char> hsync_work;
-    // pipelined FP32 decode: per-segment pulse events, pinned host copies
+    // pipelined FP32 decode: per-block pulse edges in pinned host memory
     cudaStream_t aux_stream = nullptr;   // rescue fetches while the session stream is busy
     cudaStream_t copy_stream = nullptr;  // RF copies ahead of the demod
-    cudaStream_t d2h_stream = nullptr;   // pulse events back to the host behind the demod
     cudaStream_t alt_stream = nullptr;   // odd segments, so a segment's straggler blocks overlap the next one
     cudaStream_t cap_stream = nullptr;   // origin of the pipeline graph capture
-    cudaEvent_t alt_start = nullptr, alt_end = nullptr, copy_end = nullptr, d2h_end = nullptr;
+    cudaEvent_t alt_start = nullptr, alt_end = nullptr, copy_end = nullptr, pipe_end = nullptr;
     cudaEvent_t chroma_t[2] = {nullptr, nullptr};   // stage timing: the block stage's start and end
     int demod_clusters = 0;            // clusters of the pipelined demod launches (0: one per SM pair)
     cudaGraphExec_t pipe_exec = nullptr; // captured segment pipeline
     PipeKey pipe_key{};
-    std::vector<cudaEvent_t> seg_done, seg_copied, seg_pulsed, seg_dem, seg_demod_end;
+    std::vector<cudaEvent_t> seg_copied, seg_dem;
     int nseg_max = 0;
     int64_t seg_cap = 0;                 // pulse events per segment
-    DevBuf<int64_t> seg_events, seg_total;
+    DevBuf<int64_t> seg_events;          // one segment's (scan of a stream with a full edge record)
     DevBuf<unsigned> blk_counters;       // demod block claims, one counter per launch
-    int64_t* h_events = nullptr;         // pinned [nseg_max * seg_cap]
-    int64_t* h_totals = nullptr;         // pinned [nseg_max]
+    // pinned: kEdgePad words, then max_blocks * kEdgeRecords * kEdgeWords
+    uint64_t* h_edges = nullptr;
+    uint32_t edge_tag = 0;               // of the current decode
+    bool edges_pending = false;          // a demod that writes edges may still be running
     int rescue_fetches = 0;
     int recoveries = 0;                  // field attempts that failed and were skipped past
     uint32_t launches = 0;               // kernels started by the current decode
