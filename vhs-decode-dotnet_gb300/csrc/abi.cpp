@@ -619,8 +619,7 @@ int tuned_fft_plan(vhsdecode_gb300_session* s, FastDemodParams base) {
 
 // The fused demodulator, or (VHSD_DEMOD_TIMING set) its timed diagnostic build.
 cudaError_t launch_fused(vhsdecode_gb300_session* s, FastDemodParams p, cudaStream_t st) {
-    const int clusters =
-        s->demod_clusters > 0 && p.first_claims == INT_MAX ? s->demod_clusters : s->num_sms / 2;
+    const int clusters = s->num_sms / 2;
     if (!s->demod_cycles) return launch_demod_fp32(p, clusters, st);
     p.stage_cycles = s->demod_cycles;
     return launch_demod_fp32_timed(p, clusters, st);
@@ -1127,13 +1126,19 @@ void collect_field_results(vhsdecode_gb300_session* s, cudaStream_t fs) {
 }
 
 // Segment boundaries (in blocks) of the pipelined decode: a short first
-// segment so the demod can start soon behind its RF copy, then kSegBlocks each.
-std::vector<int64_t> segment_bounds(int64_t nblocks) {
+// segment so the demod can start soon behind its RF copy, then kSegBlocks each;
+// `growing`, each after the first twice as long as the one before: pinned
+// memory is copied at more than twice the demodulator's rate, and each launch
+// costs its clusters a start (60 NTSC fields, luma, 12 launches 2.03 ms, 5
+// launches 2.00; 120 fields, 22 and 6, 3.75 and 3.66).  Pageable memory is
+// copied at about the demodulator's rate, so there the steps stay short.
+std::vector<int64_t> segment_bounds(int64_t nblocks, bool growing = false) {
     std::vector<int64_t> b{0};
-    int64_t e = std::min<int64_t>(nblocks, kFirstSegBlocks);
+    int64_t e = std::min<int64_t>(nblocks, kFirstSegBlocks), step = kSegBlocks;
     while (b.back() < nblocks) {
         b.push_back(e);
-        e = std::min<int64_t>(nblocks, e + kSegBlocks);
+        e = std::min<int64_t>(nblocks, e + step);
+        if (growing) step *= 2;
     }
     return b;
 }
@@ -1179,8 +1184,9 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
         const size_t half = (size_t)(s->num_sms / 2) * kBlock;
         p.scratch = s->scratch.p + (k & 1) * 2 * half;
         p.block_counter = s->blk_counters.p + k;
-        // one launch beside the chroma block stage: clusters for its SMs too, once they are free
-        p.first_claims = !host_input && s->demod_clusters > 0 ? s->demod_clusters : INT_MAX;
+        // beside the chroma block stage: clusters for its SMs too, once they are free
+        // (60 NTSC fields on the device, one launch: demodulated in 1.68 ms, 1.74 without them)
+        if (s->demod_clusters > 0) p.first_claims = s->demod_clusters;
         rec(s->seg_dem[(size_t)(2 * k)], ks, true);
         ck(launch_fused(s, p, ks), "demod fp32 launch");
         rec(s->seg_dem[(size_t)(2 * k + 1)], ks, true);
@@ -1323,9 +1329,8 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         }
     }
     // The chroma block stage holds an SM per CTA for its whole (latency-bound)
-    // run and is queued before the demodulator, so it has its SMs first; the
-    // demodulator is launched with only the clusters that find SMs beside it
-    // (measured 0.05 ms faster per decode than queueing clusters that wait).
+    // run and is queued before the demodulator, so it has its SMs first; only
+    // the clusters that find SMs beside it start on a block of their own.
     s->demod_clusters = 0;
     if (s->want_chroma && nblocks > 0 && !demod_only) {
         const int reserve = std::min(chroma_block_ctas(nblocks), s->num_sms / 4);
@@ -1337,7 +1342,7 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         queue_chroma_blocks(s, rf, nblocks, s->chroma_go);
     }
     // with nothing to overlap (copies), the demod runs as one launch
-    std::vector<int64_t> bounds = demod_only || !host_input ? std::vector<int64_t>{0, nblocks} : segment_bounds(nblocks);
+    std::vector<int64_t> bounds = demod_only || !host_input ? std::vector<int64_t>{0, nblocks} : segment_bounds(nblocks, graphable);
     if (nblocks == 0) bounds.assign(1, 0);
     const int nseg = (int)bounds.size() - 1;
     s->segments = (uint32_t)nseg;

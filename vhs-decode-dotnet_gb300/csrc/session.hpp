@@ -188,7 +188,7 @@ struct vhsdecode_gb300_session {
     cudaStream_t cap_stream = nullptr;   // origin of the pipeline graph capture
     cudaEvent_t alt_start = nullptr, alt_end = nullptr, copy_end = nullptr, pipe_end = nullptr;
     cudaEvent_t chroma_t[2] = {nullptr, nullptr};   // stage timing: the block stage's start and end
-    int demod_clusters = 0;            // clusters of the pipelined demod launches (0: one per SM pair)
+    int demod_clusters = 0;            // clusters of the pipelined demod that find SMs at once (0: all)
     cudaGraphExec_t pipe_exec = nullptr; // captured segment pipeline
     PipeKey pipe_key{};
     std::vector<cudaEvent_t> seg_copied, seg_dem;
