@@ -416,8 +416,7 @@ void ensure_chroma(vhsdecode_gb300_session* s) {
     }
     ck(cudaEventCreateWithFlags(&s->chroma_refined, cudaEventDisableTiming), "cudaEventCreate");
     // the block stage's stream has the highest priority: its CTAs take the
-    // first SMs that a finishing demod segment frees, ahead of the next
-    // segment's queued clusters
+    // first SMs that come free, ahead of a demodulator's queued clusters
     int least = 0, greatest = 0;
     ck(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange");
     ck(cudaStreamCreateWithPriority(&s->chroma_stream, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
@@ -1221,12 +1220,14 @@ public:
 
 private:
     // The word at `w` once it is of this decode.  The demodulator's end is
-    // looked at now and then, so that its failure ends the wait.
+    // looked at every quarter of a million polls (about half a millisecond: the
+    // look takes the driver's lock, which other threads' launches need), so
+    // that its failure ends the wait.
     uint64_t wait_word(const uint64_t* w) {
         for (unsigned spin = 1;; spin++) {
             uint64_t v = __atomic_load_n(w, __ATOMIC_ACQUIRE);
             if ((uint32_t)(v >> 32) == s_->edge_tag) return v;
-            if (spin & 1023u) continue;
+            if (spin & 0x3ffffu) continue;
             const cudaError_t q = cudaEventQuery(s_->pipe_end);
             if (q == cudaErrorNotReady) {
                 cudaGetLastError();
