@@ -384,7 +384,7 @@ def run_ours(args, world, rank, local):
     peak, peak_kind = peaks()
     avg_demod = sum(demod_ms) / len(demod_ms)
     # the same blocks as one fused-demod launch (a demod-only decode): the
-    # kernel's own rate, beside the pipelined segments' average above
+    # kernel's own rate, beside its average inside the decodes above
     single = []
     for _ in range(5):
         rs = sess.decode(None, device_ptr=d_rf.data_ptr(), count=n, demod_only=True)
@@ -393,7 +393,7 @@ def run_ours(args, world, rank, local):
     single_achieved = DEMOD_BYTES_PER_BLOCK * nblocks / (single_ms / 1e3) / 1e9
     achieved = DEMOD_BYTES_PER_BLOCK * nblocks / (avg_demod / 1e3) / 1e9
     tpb = profile_traffic_per_block(args.workload)
-    # plain FP64 baseline (one block at a time) on the same capture, one step
+    # plain FP64 baseline on the same capture, one step
     plain = None
     if not args.skip_plain:
         ps = native.Session(prof, n, precision=native.PRECISION_FP64_PLAIN, device=local, tape_format=tfmt)
@@ -458,9 +458,9 @@ def run_ours(args, world, rank, local):
                              "pipelined_segments": {
                                  "kernel_ms_sum": round(avg_demod, 4),
                                  "achieved": round(achieved, 1),
-                                 "note": "the decode's segment launches overlap on two streams; "
-                                         "their summed durations exceed the step's wall time, so "
-                                         "this is not a per-launch rate"}},
+                                 "note": "inside the decode the demod runs beside the chroma block "
+                                         "stage, and host input takes several overlapping launches, "
+                                         "so this is not the kernel's own rate"}},
                 "cpu_baseline": cpu,
                 "luma_only": other,
                 "plain_fp64": plain,

@@ -91,7 +91,7 @@ typedef enum vhsdecode_gb300_input_sample_format {
 /* Arithmetic of the block demodulator. */
 typedef enum vhsdecode_gb300_precision {
     VHSDECODE_GB300_PRECISION_FP32_FUSED = 0, /* cluster-fused FP32, FP64 sync/TBC */
-    VHSDECODE_GB300_PRECISION_FP64_PLAIN = 1  /* one block at a time, FP64 throughout */
+    VHSDECODE_GB300_PRECISION_FP64_PLAIN = 1  /* FP64 throughout, the stages as separate launches */
 } vhsdecode_gb300_precision;
 
 /* Callbacks: shapes of vhsdecode_cuda_fast_read_callback / cancel_callback (:55-62).

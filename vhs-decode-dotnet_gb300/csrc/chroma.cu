@@ -118,9 +118,10 @@ static_assert(kIirBytes % 128 == 64, "two blocks' accesses fill the 32 banks");
 // least latency (0.80 ms; 25 cycles a step); 64 is two, which holds half the
 // SMs for longer (1.2 ms).  The stage runs beside the demodulation, which
 // outlasts it in long captures: there the SMs it holds matter, in short ones
-// its latency does.  Whole luma and chroma decodes, 32 against 64: 144 blocks
-// 1.43 / 1.86 ms, 620 blocks 1.87 / 2.30, 793 blocks 2.37 / 2.47, 1011 blocks
-// 2.88 / 2.70, 1336 blocks 3.56 / 3.59 (from pinned host memory 3.82 / 3.70).
+// its latency does.  NTSC decodes with chroma, 32 against 64: 163 blocks 1.24
+// / 1.67 ms, 467 blocks 1.39 / 1.81, 793 blocks 1.89 / 1.96, 1011 blocks 2.29
+// / 2.30, 1336 blocks 2.90 / 2.88 (from pinned host memory 793 blocks 2.00 /
+// 2.12, 1011 blocks 2.46 / 2.40, 1336 blocks 3.13 / 3.03).
 // With four lanes a block and no helper warps (64 blocks a CTA, inputs read
 // by lane 0 between batches) the stage took 1.5 ms whatever the capture.
 constexpr int kBlockGroupsLow = 32;

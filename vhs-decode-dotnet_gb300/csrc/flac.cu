@@ -19,8 +19,8 @@
 //   sequential work: what bounds it is the latency of a step, about 120
 //   dependent instructions.  All four lanes read the residual (the same words
 //   of the group's ring); the predictor runs in transposed form, its taps and
-//   partial sums split over the lanes' registers, so a sample costs a lane an
-//   eighth of the 32 multiply-adds at most, no history shifts and one
+//   partial sums split over the lanes' registers, so a sample costs a lane
+//   eight of the 32 multiply-adds at most, no history shifts and one
 //   broadcast.  Frames are handed out sorted by subframe type so a warp's
 //   eight run the same path.  It checks that the subframe ends where the next
 //   frame begins and writes int16 samples (10,000 frames of 4096 samples 1.56

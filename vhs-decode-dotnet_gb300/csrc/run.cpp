@@ -385,7 +385,7 @@ VHSDECODE_GB300_API int32_t VHSDECODE_GB300_CALL vhsdecode_gb300_run(
             return fail(VHSDECODE_GB300_STATUS_INPUT_ERROR, "input shorter than one block");
 
         // FLAC bytes come in larger chunks (about 180 M samples each): a frame
-        // decodes serially on one thread, so a launch needs tens of thousands
+        // decodes serially in four lanes, so a launch needs tens of thousands
         // of frames to keep the SMs busy
         Prefetch pre(config, flac_in ? 1 : esz, flac_in ? flac_read_chunk() : kReadChunk, latch);
         std::vector<unsigned char> buf;   // source samples [buf_off, buf_off + buf.size() / esz)
