@@ -1411,7 +1411,8 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         ck(cudaEventRecord(s->ev[2], cs), "event");
     }
     finish_chroma_blocks(s, cs);
-    ck(cudaEventSynchronize(s->seg_dem[(size_t)(2 * std::max(0, nseg - 1) + 1)]), "sync");
+    // every launch: they alternate between two streams, so the last one may end before the one ahead of it
+    ck(cudaEventSynchronize(s->pipe_end), "sync");
     s->edges_pending = false;
     demod_ms = 0.0f;
     for (int k = 0; k < nseg; k++) {
