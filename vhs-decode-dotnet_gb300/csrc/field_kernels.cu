@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "pulse_bits.cuh"
+#include "tbc_stage.hpp"
 #include "kernels.h"
 
 namespace vhsd {
@@ -1568,15 +1569,10 @@ __global__ void __launch_bounds__(kTbcFastMaxThreads, 3) k_tbc_fast(const float*
     const int lane = threadIdx.x & 31;
     const int q = lane >> 2, sub = lane & 3;
     float* wrow = weights + (threadIdx.x & ~31) * kTapRow;   // the warp's 32 rows
-    // The stretch [lo, lo + len) of the span, four floats at a time, that the
-    // line's taps (positions run one way along the line) and load_taps's
-    // neighbours lie in.  A line whose taps leave the span or the stage (its
-    // locations are no line's) is read from global memory tap by tap.
-    const int first = tap_pos(c, p.x0).ci - 7, last = tap_pos(c, kx1 - 1).ci - 7;
-    const int lo = min(first, last) & ~3;
-    const int len = ((max(first, last) + 19 - lo) + 3) & ~3;
+    const TbcStretch part = tbc_stretch(tap_pos(c, p.x0).ci, tap_pos(c, kx1 - 1).ci, n32, stage_cap);
+    const bool staged = part.staged;
+    const int lo = part.lo, len = part.len;
     const int lo2 = lo - ((lo + chroma.offset) & 3);   // the same for the chroma, on its rows' alignment
-    const bool staged = min(first, last) >= 0 && len > 0 && len + 4 <= stage_cap && lo + len <= n32;
     if (staged) {
         if (!kRows)
             for (int i = 4 * threadIdx.x; i < len; i += 4 * blockDim.x)
