@@ -606,8 +606,7 @@ __device__ __forceinline__ void sync_bits(Shared& sh, float2 q, int base, int64_
 // the tag instead of a fence ahead of the header: a fence to the system's scope
 // cost another 5,000 cycles a block, one to the device's 2,000.  Called by
 // every thread, after a barrier behind sync_bits.
-__device__ __noinline__ void write_edges(Shared& sh, const FastDemodParams& p, unsigned tag32, int64_t blk,
-                                         int rank) {
+__device__ __noinline__ void write_edges(Shared& sh, const FastDemodParams& p, int64_t blk, int rank) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = 2 * (tid >> 8) + rank;
     const int n = c * 8192 + 32 * (tid & 255);
@@ -660,7 +659,7 @@ __device__ __noinline__ void write_edges(Shared& sh, const FastDemodParams& p, u
     }
     if (extra && lane == head) e |= 1u << b_first;
     unsigned o = off + (unsigned)(incl - pc) + (extra && lane > head ? 1u : 0u);
-    const unsigned long long tag = (unsigned long long)tag32 << 32;
+    const unsigned long long tag = (unsigned long long)sh.edge_tag << 32;
     unsigned long long* rec = p.edges + ((blk + p.first_block) * kEdgeRecords + c) * (int64_t)kEdgeWords;
     auto store = [](unsigned long long* at, unsigned long long v) {
         asm volatile("st.relaxed.sys.global.u64 [%0], %1;\n" ::"l"(at), "l"(v) : "memory");
@@ -792,8 +791,7 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         }
     }
     if constexpr (!BATCHED) {
-        if (tid == 0 && pk.edges)
-            sh.edge_tag = pk.edge_tag_at ? *reinterpret_cast<const volatile unsigned*>(pk.edge_tag_at) : pk.edge_tag;
+        if (tid == 0 && pk.edges) sh.edge_tag = *reinterpret_cast<const volatile unsigned*>(pk.edge_tag_at);
     }
     // Blocks: each cluster starts on block cluster_id (those that may start
     // late, from first_claims on, claim that one too) and then claims the next
@@ -1112,9 +1110,11 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
                 }
             }
         }
-        if (p.edges) {
-            __syncthreads();
-            write_edges(sh, p, BATCHED ? p.edge_tag : sh.edge_tag, blk, rank);
+        if constexpr (!BATCHED) {
+            if (pk.edges) {
+                __syncthreads();
+                write_edges(sh, pk, blk, rank);
+            }
         }
         VHSD_MARK(17);
         if (sub) {

@@ -60,16 +60,15 @@ struct FastDemodParams {
     float sync_thr;
     // optional pulse edges of each block, in pinned host memory (null: not
     // written): per stream block four records of kEdgeWords words, one for each
-    // 8192-sample chunk.  A word's upper half is the decode's tag, *edge_tag_at
-    // (or edge_tag where that is null), so the host tells a word of this
-    // decode from an older one.  Word 0, written last, is the chunk's header
-    // (edge_header below); words 1.. hold its edges in stream order: 2 x the
-    // position in the block's 30720 stream samples, + 1 where the signal rises
-    // through sync_thr.  The chunk's first non-NaN sample makes no edge here:
-    // the state before it is the previous chunk's, which the host knows.
+    // 8192-sample chunk.  A word's upper half is the decode's tag, *edge_tag_at,
+    // so the host tells a word of this decode from an older one.  Word 0 is the
+    // chunk's header (kEdgeWords below); words 1.. hold its edges in stream
+    // order: 2 x the position in the block's 30720 stream samples, + 1 where the
+    // signal rises through sync_thr.  The chunk's first non-NaN sample makes no
+    // edge here: the state before it is the previous chunk's, which the host
+    // knows.  Not in a batched launch, whose windows are scanned afterwards.
     unsigned long long* edges;
     const unsigned* edge_tag_at;
-    unsigned edge_tag;
     // diagnostics only (launch_demod_fp32_timed): per-rank cycle sums of the
     // kernel's stages, [rank * kDemodStages + stage]
     unsigned long long* stage_cycles;
