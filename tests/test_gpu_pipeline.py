@@ -25,3 +25,78 @@ def test_last_launch_ends_before_the_one_ahead(gpu, mhz):
             r = s.decode(pinned.numpy())
             assert (r.fields, r.blocks, r.segments) == (0, 41, 2)
             assert r.repaired_blocks > 0 and r.demod_ms > 0.0
+
+
+def _long_pulses(rf, cfg):
+    """`rf` with hsync pulses of 9 us on five lines of every field."""
+    from vhsd_gb300 import synth
+    g = synth._geometry(cfg.system)
+    line = g["line_us"] * cfg.fs / 1e6
+    out = rf.copy()
+    n = int(6e-6 * cfg.fs)
+    tip = np.round(8000.0 * np.cos(2 * np.pi * np.arange(n) * (cfg.ire0 + cfg.hz_ire * cfg.vsync_ire) / cfg.fs))
+    for field in range(int(cfg.fields) + 1):
+        for k in (60, 100, 140, 180, 220):
+            at = int((cfg.lead_lines + field * (g["lines"] // 2 + 1) + k) * line + 3e-6 * cfg.fs)
+            if at + n <= len(out):
+                out[at:at + n] = tip
+    return out
+
+
+def _rescues(capfd):
+    return [int(line.split("rescue_fetches=")[1].split()[0]) for line in capfd.readouterr().err.splitlines()
+            if "rescue_fetches=" in line]
+
+
+def test_rescue_reads_finished_blocks(gpu, monkeypatch, capfd):
+    # the long-hsync rescue reads sync samples of blocks that the running
+    # demodulator has finished: the same fields, lines and pictures whichever way
+    # the capture comes in, also right after a decode of another one (whose
+    # samples an early read would find), and the fields of the double-precision
+    # decode, which reads after its whole demodulation
+    import torch
+    from vhsd_gb300 import native, synth
+    monkeypatch.setenv("VHSD_STAGE_TIMING", "1")
+    cfg = synth.ntsc_vhs(fields=12, seed=11, snr_db=40.0)
+    clean, _ = synth.generate(cfg)
+    rf = _long_pulses(clean, cfg)
+    pinned, dev = torch.from_numpy(rf).pin_memory(), torch.from_numpy(rf).cuda()
+    with native.Session(native.PROFILE_NTSC, len(rf), precision=native.PRECISION_FP64_PLAIN) as s:
+        r = s.decode(rf)
+        spans = [(s.field(i).span_start, bool(s.field(i).is_first_field)) for i in range(r.fields)]
+    assert len(spans) >= 11
+    capfd.readouterr()
+    want = None
+    with native.Session(native.PROFILE_NTSC, len(rf)) as s:
+        for source in ("device", "pinned", "pageable") * 4:
+            s.decode(clean)
+            capfd.readouterr()
+            if source == "device":
+                r = s.decode(None, device_ptr=dev.data_ptr(), count=len(rf))
+            else:
+                r = s.decode(pinned.numpy() if source == "pinned" else rf)
+            assert _rescues(capfd)[0] > 0
+            assert [(s.field(i).span_start, bool(s.field(i).is_first_field)) for i in range(r.fields)] == spans
+            got = (s.tbc(), np.concatenate([s.lines(i) for i in range(r.fields)]))
+            want = want or got
+            assert all(np.array_equal(a, b) for a, b in zip(got, want)), source
+
+
+def test_rescue_does_not_wait_for_the_demodulator(gpu, monkeypatch, capfd):
+    # 3000 blocks on the device, one launch, the first field only: its blocks
+    # and the rescue's samples are there after a few of the 40 rounds of blocks
+    import torch
+    from vhsd_gb300 import native, synth
+    monkeypatch.setenv("VHSD_STAGE_TIMING", "1")
+    cfg = synth.ntsc_vhs(fields=4, seed=12, snr_db=40.0)
+    rf = np.resize(_long_pulses(synth.generate(cfg)[0], cfg), 2999 * STRIDE + BLOCK)
+    dev = torch.from_numpy(rf).cuda()
+    with native.Session(native.PROFILE_NTSC, len(rf)) as s:
+        times = []
+        for _ in range(5):
+            capfd.readouterr()
+            r = s.decode(None, device_ptr=dev.data_ptr(), count=len(rf), max_fields=1)
+            assert r.fields == 1 and r.segments == 1 and _rescues(capfd)[0] > 0
+            times.append((r.host_ms, r.demod_ms))
+        host, demod = np.median(times, axis=0)
+        assert host < 0.5 * demod, (host, demod)

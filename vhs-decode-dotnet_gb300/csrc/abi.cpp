@@ -213,10 +213,11 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
         s->seg_cap = kSegBlocks * kStride / 64 + 4096;
         s->seg_events.alloc((size_t)s->seg_cap);
         s->blk_counters.alloc((size_t)s->nseg_max + 1);   // one per segment launch, the last for run_demod
-        const size_t edge_bytes =
-            (kEdgePad + (size_t)std::max<int64_t>(1, s->max_blocks) * kEdgeRecords * kEdgeWords) * sizeof(uint64_t);
-        ck(cudaHostAlloc((void**)&s->h_edges, edge_bytes, cudaHostAllocDefault), "cudaHostAlloc");
-        ck(cudaMemset(s->h_edges, 0, edge_bytes), "memset");   // no decode has tag 0
+        const size_t edge_blocks = (size_t)std::max<int64_t>(1, s->max_blocks);
+        s->edge_words = kEdgePad + edge_blocks * kEdgeRecords * kEdgeWords + (size_t)s->nseg_max * (s->num_sms / 2);
+        ck(cudaHostAlloc((void**)&s->h_edges, s->edge_words * sizeof(uint64_t), cudaHostAllocDefault), "cudaHostAlloc");
+        ck(cudaMemset(s->h_edges, 0, s->edge_words * sizeof(uint64_t)), "memset");   // no decode has tag 0
+        s->h_progress = s->h_edges + kEdgePad + edge_blocks * kEdgeRecords * kEdgeWords;
         s->seg_copied.resize((size_t)s->nseg_max);
         s->seg_dem.resize((size_t)s->nseg_max * 2);
         for (auto& e : s->seg_copied) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
@@ -712,16 +713,18 @@ void run_demod(vhsdecode_gb300_session* s, const int16_t* rf_dev, int64_t nblock
 // Pulse events of the stitched stream in stream order.  upto(pos) returns once
 // every event before stream position pos is in `events` (the pipelined decode
 // waits there for the segment that finalises pos).
+// ready(pos, len) returns once a copy may read stream samples [pos, pos + len),
+// whose events are in already (unset: once the events are in).
 struct EventFeed {
     std::vector<int64_t> events;
     std::function<void(int64_t)> upto;
+    std::function<void(int64_t, int64_t)> ready;
 };
 
 // TbcFieldSequenceDecodeEngine order (Core/Decode/TbcFieldSequenceDecodeEngine.cs:442-560):
 // resolve the next field span, take its pulses, run the control plane, step by
 // the next-field offset.  The long-hsync rescue reads the sync reference of a
-// finished span on the auxiliary stream, so it waits for the demodulation but
-// for no other queued work.
+// finished span on the auxiliary stream, so it never waits behind queued work.
 template <typename T>
 void host_field_loop(vhsdecode_gb300_session* s, const T* sync, int64_t stream_len, uint32_t max_fields,
                      EventFeed& feed, uint32_t& stop_reason, const std::atomic<bool>* cancel,
@@ -750,8 +753,7 @@ void host_field_loop(vhsdecode_gb300_session* s, const T* sync, int64_t stream_l
                                              min_len, max_len);
         RefFetch fetch = [&](int64_t start, int64_t len, std::vector<double>& out) {
             tmp.resize((size_t)len);
-            // an edge record says nothing about the sync samples of its block
-            if (s->edges_pending) ck(cudaStreamWaitEvent(s->aux_stream, s->pipe_end, 0), "rescue fetch");
+            if (feed.ready) feed.ready(s0 + start, len);
             ck(cudaMemcpyAsync(tmp.data(), sync + s0 + start, (size_t)len * sizeof(T),
                                cudaMemcpyDeviceToHost, s->aux_stream), "rescue fetch");
             ck(cudaStreamSynchronize(s->aux_stream), "rescue fetch");
@@ -1183,6 +1185,7 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
         const size_t half = (size_t)(s->num_sms / 2) * kBlock;
         p.scratch = s->scratch.p + (k & 1) * 2 * half;
         p.block_counter = s->blk_counters.p + k;
+        p.progress = reinterpret_cast<unsigned long long*>(s->h_progress) + (size_t)k * (s->num_sms / 2);
         // beside the chroma block stage: clusters for its SMs too, once they are free
         // (60 NTSC fields on the device, one launch: demodulated in 1.68 ms, 1.74 without them)
         if (s->demod_clusters > 0) p.first_claims = s->demod_clusters;
@@ -1205,8 +1208,8 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
 // once the demodulation queued on `cs` is over.
 class EdgeReader {
 public:
-    EdgeReader(vhsdecode_gb300_session* s, int64_t nblocks, cudaStream_t cs)
-        : s_(s), nblocks_(nblocks), cs_(cs) {}
+    EdgeReader(vhsdecode_gb300_session* s, const std::vector<int64_t>& bounds, cudaStream_t cs)
+        : s_(s), bounds_(bounds), nblocks_(bounds.back()), cs_(cs) {}
     void upto(int64_t pos, std::vector<int64_t>& events) {
         while (next_ * kStride < pos && next_ < nblocks_) {
             if (!take_block(events)) {
@@ -1218,15 +1221,28 @@ public:
         }
     }
 
+    // Returns once a copy may read stream samples [pos, pos + len), whose blocks'
+    // edges have been taken.
+    void ready(int64_t pos, int64_t len) {
+        __atomic_store_n(reinterpret_cast<uint32_t*>(s_->h_edges) + kEdgeAsk, s_->edge_tag, __ATOMIC_RELEASE);
+        for (int64_t b = pos / kStride; b * kStride < pos + len; b++) {
+            const size_t launch = (size_t)(std::upper_bound(bounds_.begin(), bounds_.end(), b) - bounds_.begin()) - 1;
+            const uint64_t* at = s_->h_progress + launch * (size_t)(s_->num_sms / 2) + ((uint32_t)*record(b) >> 24);
+            if ((uint32_t)wait_word(at, (uint32_t)b + 1) == kEdgeLeft)
+                ck(cudaEventSynchronize(s_->seg_dem[2 * launch + 1]), "segment wait");
+        }
+    }
+
 private:
-    // The word at `w` once it is of this decode.  The demodulator's end is
-    // looked at every quarter of a million polls (about half a millisecond: the
-    // look takes the driver's lock, which other threads' launches need), so
-    // that its failure ends the wait.
-    uint64_t wait_word(const uint64_t* w) {
+    // The word at `w` once it is of this decode and its lower half `least` or
+    // more.  The demodulator's end is looked at every quarter of a million polls
+    // (about half a millisecond: the look takes the driver's lock, which other
+    // threads' launches need), so that its failure ends the wait.
+    uint64_t wait_word(const uint64_t* w, uint32_t least = 0) {
+        auto here = [&](uint64_t v) { return (uint32_t)(v >> 32) == s_->edge_tag && (uint32_t)v >= least; };
         for (unsigned spin = 1;; spin++) {
             uint64_t v = __atomic_load_n(w, __ATOMIC_ACQUIRE);
-            if ((uint32_t)(v >> 32) == s_->edge_tag) return v;
+            if (here(v)) return v;
             if (spin & 0x3ffffu) continue;
             const cudaError_t q = cudaEventQuery(s_->pipe_end);
             if (q == cudaErrorNotReady) {
@@ -1235,25 +1251,28 @@ private:
             }
             ck(q, "segment wait");
             v = __atomic_load_n(w, __ATOMIC_ACQUIRE);
-            if ((uint32_t)(v >> 32) == s_->edge_tag) return v;
+            if (here(v)) return v;
             throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "a block's pulse edges are missing");
         }
     }
+    const uint64_t* record(int64_t block) const {
+        return s_->h_edges + kEdgePad + (size_t)block * kEdgeRecords * kEdgeWords;
+    }
     bool take_block(std::vector<int64_t>& events) {
-        const uint64_t* rec = s_->h_edges + kEdgePad + (size_t)next_ * kEdgeRecords * kEdgeWords;
+        const uint64_t* rec = record(next_);
         const int64_t base = 2 * next_ * kStride;
         for (int c = 0; c < kEdgeRecords; c++, rec += kEdgeWords) {
             // two blocks on: the records lie a kilobyte apart
             if (next_ + 2 < nblocks_) __builtin_prefetch(rec + 2 * kEdgeRecords * kEdgeWords);
             const uint32_t h = (uint32_t)wait_word(rec);
-            const int count = (int)(h & 16383u);
+            const int count = (int)(h & 255u);
             if (count > kEdgeCap) return false;
-            if (!((h >> 29) & 1u)) continue;
-            const bool first = (h >> 27) & 1u;
+            if (!((h >> 23) & 1u)) continue;
+            const bool first = (h >> 21) & 1u;
             if (first != state_)
-                events.push_back(base + 2 * (c * (kBlock / 4) + (int64_t)((h >> 14) & 8191u) - kCut - 32) + (first ? 0 : 1));
+                events.push_back(base + 2 * (c * (kBlock / 4) + (int64_t)((h >> 8) & 8191u) - kCut - 32) + (first ? 0 : 1));
             for (int i = 1; i <= count; i++) events.push_back(base + (int64_t)(uint32_t)wait_word(rec + i));
-            state_ = (h >> 28) & 1u;
+            state_ = (h >> 22) & 1u;
         }
         return true;
     }
@@ -1279,6 +1298,7 @@ private:
         }
     }
     vhsdecode_gb300_session* s_;
+    const std::vector<int64_t>& bounds_;   // the launches' blocks
     int64_t nblocks_, next_ = 0;
     cudaStream_t cs_;
     bool state_ = false;
@@ -1352,7 +1372,7 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
         // a demod that an earlier decode left behind (it failed) reads the tag when it starts
         if (s->edges_pending) ck(cudaStreamSynchronize(cs), "sync");
         if (++s->edge_tag == 0) {   // 2^32 decodes on: no word may look new
-            std::memset(s->h_edges, 0, (kEdgePad + (size_t)s->max_blocks * kEdgeRecords * kEdgeWords) * sizeof(uint64_t));
+            std::memset(s->h_edges, 0, s->edge_words * sizeof(uint64_t));
             s->edge_tag = 1;
         }
         __atomic_store_n(reinterpret_cast<uint32_t*>(s->h_edges), s->edge_tag, __ATOMIC_RELEASE);
@@ -1391,8 +1411,9 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     if (!demod_only && nblocks > 0) {
         auto t0 = std::chrono::steady_clock::now();
         EventFeed feed;
-        EdgeReader edges(s, nblocks, cs);
+        EdgeReader edges(s, bounds, cs);
         feed.upto = [&](int64_t pos) { edges.upto(pos, feed.events); };
+        feed.ready = [&](int64_t pos, int64_t len) { edges.ready(pos, len); };
         // The field kernels run as one batch over all fields after the host
         // loop: batches launched from the host loop while the closing segments
         // demodulate were slower (host launch and copy time lands on the

@@ -196,6 +196,7 @@ struct Shared {
     int flag;
     unsigned edge_tag;       // the decode's tag of the pulse edges
     unsigned edge_sum[T / 32];   // each warp's edges, and its first and last state
+    uint4 ask;               // rank 1: the host's request for progress (its first word)
     long long next_blk[2];   // the cluster's next block, by iteration parity
     int next_job[2];         // batched launch: the next block's window
     int cur_job;
@@ -672,7 +673,27 @@ __device__ __noinline__ void write_edges(Shared& sh, const FastDemodParams& p, i
         o++;
     }
     if ((tid & 255) == 0)
-        store(rec, tag | count | (first_at << 14) | (first_state << 27) | (state << 28) | (known << 29));
+        store(rec, tag | min(count, kEdgeCap + 1u) | (first_at << 8) | (first_state << 21) | (state << 22) | (known << 23) |
+                       ((blockIdx.x >> 1) << 24));
+}
+
+// FastDemodParams::progress, by rank 1's first thread (rank 0's claims blocks).
+// The host's request is copied to shared memory in one block and looked at in
+// the next: while captures move, a copy from the host takes longer than a
+// transform.
+__device__ __forceinline__ void ask_progress(uint4* to, const unsigned* ask) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(to)),
+                 "l"(ask) : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+// Behind a cluster barrier after the stores that it answers for (the fence is
+// cumulative).  60 NTSC fields, whole calls from the device / pinned, luma: a
+// fence behind every block cost 0.4 / 0.6 % (the device's scope) or 0.7 / 1.2 %
+// (the system's), one as every cluster ends 1 % of a decode with chroma from
+// pinned memory; with fences only once the host asks, nothing.
+__device__ __forceinline__ void publish_progress(unsigned tag, unsigned long long* to, unsigned at) {
+    if (at != kEdgeLeft) __threadfence_system();
+    asm volatile("st.relaxed.sys.global.u64 [%0], %1;\n" ::"l"(to), "l"((unsigned long long)tag << 32 | at) : "memory");
 }
 
 // Next block's RF (32768 int16 = 64 KB, both halves) into `dst` with
@@ -791,6 +812,7 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         }
     }
     if constexpr (!BATCHED) {
+        if (tid == 0) sh.ask.x = 0;
         if (tid == 0 && pk.edges) sh.edge_tag = *reinterpret_cast<const volatile unsigned*>(pk.edge_tag_at);
     }
     // Blocks: each cluster starts on block cluster_id (those that may start
@@ -832,6 +854,10 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         // ---------------- stage 1: RF forward FFT (packed, DIF split) -----
         prefetch_wait();
         __syncthreads();
+        if constexpr (!BATCHED) {
+            if (rank == 1 && tid == 0 && pk.edges && sh.ask.x == sh.edge_tag)
+                publish_progress(sh.edge_tag, pk.progress + (blockIdx.x >> 1), (unsigned)(blk + pk.first_block));
+        }
         if constexpr (TIMED) t_mark = clock64();
         if (f32_in) load_rf_f32(buf, p.rf_f32 + (blk + p.first_block) * (int64_t)S, rank, sh.tw, tid);
         else load_rf(buf, rf_smem, rank, sh.tw, tid);
@@ -842,6 +868,9 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         fft8192<false, 1, PLAN>(buf, sh.tw, tid);
         VHSD_MARK(1);
         prefetch_wait();
+        if constexpr (!BATCHED) {
+            if (rank == 1 && tid == 0 && pk.edges) ask_progress(&sh.ask, pk.edge_tag_at + kEdgeAsk);
+        }
         __syncthreads();
         // X * RfVideo * Hilbert / N  (Hilbert: 1 at 0 and N/2, 2 between)
         {
@@ -1200,6 +1229,12 @@ vhsd_demod_fp32_kernel(FastDemodParams pk) {
         }
         g = nxt;
         par ^= 1;
+    }
+    if constexpr (!BATCHED) {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");   // the last request
+        if (rank == 1 && tid == 0 && pk.edges)
+            publish_progress(sh.edge_tag, pk.progress + (blockIdx.x >> 1),
+                             sh.ask.x == sh.edge_tag ? kEdgeEnded : kEdgeLeft);
     }
 }
 

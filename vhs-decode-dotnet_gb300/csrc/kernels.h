@@ -69,6 +69,13 @@ struct FastDemodParams {
     // knows.  Not in a batched launch, whose windows are scanned afterwards.
     unsigned long long* edges;
     const unsigned* edge_tag_at;
+    // with edges, in pinned host memory too.  An edge record says nothing about
+    // the streams and bits of its block, only which cluster took it.  Once the
+    // host has stored the tag in edge_tag_at[kEdgeAsk], every cluster keeps a
+    // stream block in progress[its index]: what it took below can be read by a
+    // copy.  A cluster that ends leaves kEdgeEnded there, or kEdgeLeft where it
+    // saw no request: its blocks can be read once the launch has ended.
+    unsigned long long* progress;
     // diagnostics only (launch_demod_fp32_timed): per-rank cycle sums of the
     // kernel's stages, [rank * kDemodStages + stage]
     unsigned long long* stage_cycles;
@@ -85,12 +92,16 @@ constexpr int kDemodStages = 20;
 // lines (seven edges; fourteen in a vertical interval), the 0.5 MHz sync
 // filter passes at most about a hundred crossings a chunk; a chunk with more
 // is left to the pulse scan of the whole stream.  The lower half of a header:
-// bits 0-13 the chunk's edges, 14-26 its first non-NaN sample, 27 and 28 the
-// states of its first and last one (1: v <= threshold), 29 whether it has any.
+// bits 0-7 the chunk's edges (kEdgeCap + 1: more than it holds), 8-20 its first
+// non-NaN sample, 21 and 22 the states of its first and last one (1: v <=
+// threshold), 23 whether it has any, 24-31 the cluster's index in its launch
+// (the 152 SMs hold 76).
 constexpr int kEdgeWords = 128;
 constexpr int kEdgeCap = kEdgeWords - 1;
 constexpr int kEdgeRecords = 4;   // per block
-constexpr int kEdgePad = 16;      // words ahead of the records: the first holds the decode's tag
+constexpr int kEdgePad = 16;      // words ahead of the records: the first holds the decode's tag,
+constexpr int kEdgeAsk = 16;      //   the one 64 bytes on the same when the host asks for progress
+constexpr unsigned kEdgeLeft = 0xfffffffeu, kEdgeEnded = 0xffffffffu;
 // Radix plans the fused kernel is compiled for (8192-point plan | 16384-point
 // plan << 2): 16x16x32 | 16x32x32, 32x16x16 | 16x32x32, 16x16x32 | 32x32x16,
 // 32x16x16 | 32x32x16.  The other plans of the transforms (16x32x16, 8x32x32;

@@ -196,8 +196,11 @@ struct vhsdecode_gb300_session {
     int64_t seg_cap = 0;                 // pulse events per segment
     DevBuf<int64_t> seg_events;          // one segment's (scan of a stream with a full edge record)
     DevBuf<unsigned> blk_counters;       // demod block claims, one counter per launch
-    // pinned: kEdgePad words, then max_blocks * kEdgeRecords * kEdgeWords
+    // pinned: kEdgePad words, max_blocks * kEdgeRecords * kEdgeWords of records,
+    // nseg_max * num_sms / 2 progress words
     uint64_t* h_edges = nullptr;
+    uint64_t* h_progress = nullptr;
+    size_t edge_words = 0;
     uint32_t edge_tag = 0;               // of the current decode
     bool edges_pending = false;          // a demod that writes edges may still be running
     int rescue_fetches = 0;
