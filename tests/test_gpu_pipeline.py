@@ -100,3 +100,53 @@ def test_rescue_does_not_wait_for_the_demodulator(gpu, monkeypatch, capfd):
             times.append((r.host_ms, r.demod_ms))
         host, demod = np.median(times, axis=0)
         assert host < 0.5 * demod, (host, demod)
+
+
+@pytest.mark.parametrize("mhz,fields,crowds,segments", [
+    (40.0, 10, [(60, 2)], 1),                        # inside the second segment of blocks (of 40, 128 and the rest)
+    (40.0, 10, [(20, 1), (200, 2)], 2),              # the first and the third
+    (40.0, 10, [(165, 6)], 2),                       # across the end of the second
+    (20.0, 14, [(10, 2), (36, 7)], 2),               # two in one segment, the later one across its end
+])
+def test_crowded_blocks_scan_their_segment(gpu, mhz, fields, crowds, segments):
+    # blocks with more edges than a record holds (a 0.4 MHz square wave around
+    # the threshold: 160 a chunk at 40 MSPS, 320 at 20): the rest of their segment
+    # is scanned on the device, two kernels each, the others keep their records.
+    # The fields are those of the double-precision decode's scan of its own
+    # stream, whichever way the capture comes in.
+    import torch
+    from oracle import formats
+    from vhsd_gb300 import native, synth
+    clean, _ = synth.generate(synth.ntsc_vhs(fs=mhz * 1e6, fields=fields, seed=21, snr_db=40.0))
+    fmt = formats.get("NTSC")["sys"]
+    rf = clean.copy()
+    for block, count in crowds:
+        t = np.arange(count * STRIDE)
+        ire = np.where((t * 0.8e6 / (mhz * 1e6)).astype(np.int64) % 2 == 0, -60.0, 20.0)
+        wave = 8000.0 * np.cos(2 * np.pi * np.cumsum(fmt["ire0"] + fmt["hz_ire"] * ire) / (mhz * 1e6))
+        rf[block * STRIDE + 8000:block * STRIDE + 8000 + len(t)] = np.round(wave)
+    pinned, dev = torch.from_numpy(rf).pin_memory(), torch.from_numpy(rf).cuda()
+
+    def spans(s, r):
+        return [(s.field(i).span_start, bool(s.field(i).is_first_field)) for i in range(r.fields)]
+
+    with native.Session(native.PROFILE_NTSC, len(rf), sample_rate_mhz=mhz,
+                        precision=native.PRECISION_FP64_PLAIN) as s:
+        want = spans(s, s.decode(rf))
+    assert len(want) >= fields // 2
+    pictures = None
+    with native.Session(native.PROFILE_NTSC, len(rf), sample_rate_mhz=mhz) as s:
+        for source in ("device", "pinned", "pageable"):
+            launches = []
+            for x in (clean, rf):
+                if x is rf and source == "device":
+                    r = s.decode(None, device_ptr=dev.data_ptr(), count=len(rf))
+                else:
+                    r = s.decode(pinned.numpy() if x is rf and source == "pinned" else x)
+                assert r.fields > 0
+                launches.append(r.kernel_launches - r.segments)
+            assert launches[1] - launches[0] == 2 * segments, source
+            assert spans(s, r) == want, source
+            got = (s.tbc(), np.concatenate([s.lines(i) for i in range(r.fields)]))
+            pictures = pictures or got
+            assert all(np.array_equal(a, b) for a, b in zip(got, pictures)), source

@@ -1203,21 +1203,28 @@ void enqueue_pipeline(vhsdecode_gb300_session* s, const int16_t* rf, uint64_t n,
 
 // Pulse events of the stitched stream as the demodulator finishes its blocks:
 // the blocks' edge records (FastDemodParams::edges) are taken in stream order,
-// each joined to the state that the one before ends in.  A record with more
-// edges than it holds sends the whole stream through the pulse scan instead,
-// once the demodulation queued on `cs` is over.
+// each joined to the state that the one before ends in.  From a block with more
+// edges than its records hold the rest of its segment (segment_bounds) is
+// scanned instead, once it is demodulated.
 class EdgeReader {
 public:
-    EdgeReader(vhsdecode_gb300_session* s, const std::vector<int64_t>& bounds, cudaStream_t cs)
-        : s_(s), bounds_(bounds), nblocks_(bounds.back()), cs_(cs) {}
+    EdgeReader(vhsdecode_gb300_session* s, const std::vector<int64_t>& bounds)
+        : s_(s), bounds_(bounds), segs_(segment_bounds(bounds.back())), nblocks_(bounds.back()) {}
     void upto(int64_t pos, std::vector<int64_t>& events) {
         while (next_ * kStride < pos && next_ < nblocks_) {
-            if (!take_block(events)) {
-                scan_stream(events);
-                next_ = nblocks_;
-                return;
+            if (next_ == segs_[seg_ + 1]) {
+                seg_++;
+                seg_events_ = events.size();
             }
-            next_++;
+            const size_t at = events.size();
+            const bool state = state_;
+            if (take_block(events)) {
+                next_++;
+            } else {
+                events.resize(at);
+                state_ = state;
+                scan_segment(events);
+            }
         }
     }
 
@@ -1276,31 +1283,36 @@ private:
         }
         return true;
     }
-    void scan_stream(std::vector<int64_t>& events) {
-        ck(cudaStreamSynchronize(cs_), "segment wait");
-        events.clear();
-        const std::vector<int64_t> bounds = segment_bounds(nblocks_);
-        for (size_t k = 0; k + 1 < bounds.size(); k++) {
-            ck(launch_pulse_bits_range(s_->sync_cond.p, s_->sync_hold.p, bounds[k] * kStride, bounds[k + 1] * kStride,
-                                       s_->pc_counts.p, s_->pc_offsets.p, s_->seg_events.p, s_->seg_cap,
-                                       s_->pc_total.p, cs_), "pulse launch");
-            s_->launches += kPulseKernels;
-            int64_t total = 0;
-            ck(cudaMemcpyAsync(&total, s_->pc_total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, cs_), "d2h");
-            ck(cudaStreamSynchronize(cs_), "sync");
-            if (total > s_->seg_cap)
-                throw Failure(VHSDECODE_GB300_STATUS_DECODE_ERROR, "sync pulse event capacity exceeded");
-            const size_t at = events.size();
-            events.resize(at + (size_t)total);
-            if (total)
-                ck(cudaMemcpy(events.data() + at, s_->seg_events.p, (size_t)total * sizeof(int64_t),
-                              cudaMemcpyDeviceToHost), "d2h events");
+    // Blocks next_ and on of the segment by the pulse scan of their bits.  Its
+    // CTAs find no SM while the demodulator holds all of them, so it waits for
+    // the launches that the blocks, and the states before them, come from.
+    void scan_segment(std::vector<int64_t>& events) {
+        const int64_t end = segs_[seg_ + 1];
+        for (size_t k = 0; bounds_[k] < end; k++) ck(cudaEventSynchronize(s_->seg_dem[2 * k + 1]), "segment wait");
+        cudaStream_t as = s_->aux_stream;
+        ck(launch_pulse_bits_range(s_->sync_cond.p, s_->sync_hold.p, next_ * kStride, end * kStride, s_->pc_counts.p,
+                                   s_->pc_offsets.p, s_->seg_events.p, s_->seg_cap, s_->pc_total.p, as), "pulse launch");
+        s_->launches += kPulseKernels;
+        int64_t total = 0;
+        ck(cudaMemcpyAsync(&total, s_->pc_total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, as), "d2h");
+        ck(cudaStreamSynchronize(as), "sync");
+        const size_t at = events.size();
+        if ((int64_t)(at - seg_events_) + total > s_->seg_cap)
+            throw Failure(VHSDECODE_GB300_STATUS_DECODE_ERROR, "sync pulse event capacity exceeded");
+        events.resize(at + (size_t)total);
+        if (total) {
+            ck(cudaMemcpyAsync(events.data() + at, s_->seg_events.p, (size_t)total * sizeof(int64_t),
+                               cudaMemcpyDeviceToHost, as), "d2h events");
+            ck(cudaStreamSynchronize(as), "sync");
+            state_ = !(events.back() & 1);   // below the threshold after a fall
         }
+        next_ = end;
     }
     vhsdecode_gb300_session* s_;
     const std::vector<int64_t>& bounds_;   // the launches' blocks
+    const std::vector<int64_t> segs_;
     int64_t nblocks_, next_ = 0;
-    cudaStream_t cs_;
+    size_t seg_ = 0, seg_events_ = 0;      // the segment of next_, the events before it
     bool state_ = false;
 };
 
@@ -1411,7 +1423,7 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     if (!demod_only && nblocks > 0) {
         auto t0 = std::chrono::steady_clock::now();
         EventFeed feed;
-        EdgeReader edges(s, bounds, cs);
+        EdgeReader edges(s, bounds);
         feed.upto = [&](int64_t pos) { edges.upto(pos, feed.events); };
         feed.ready = [&](int64_t pos, int64_t len) { edges.ready(pos, len); };
         // The field kernels run as one batch over all fields after the host

@@ -88,10 +88,12 @@ struct FastDemodParams {
     int batch_njobs;
 };
 constexpr int kDemodStages = 20;
-// Edge records: a header and up to kEdgeCap edges.  A chunk holds about three
-// lines (seven edges; fourteen in a vertical interval), the 0.5 MHz sync
-// filter passes at most about a hundred crossings a chunk; a chunk with more
-// is left to the pulse scan of the whole stream.  The lower half of a header:
+// Edge records: a header and up to kEdgeCap edges.  A chunk of 8192 samples is
+// 205 us at 40 MSPS, about three lines (seven edges; fourteen in a vertical
+// interval), and 410 us at 20.  The sync filter passes 0.5 MHz, two crossings a
+// microsecond at most: noise of a blank tape at 10 to 40 MSPS stays below the
+// record's size, a 0.4 MHz wave around the threshold does not (160 at 40 MSPS).
+// Such a chunk is left to the pulse scan.  The lower half of a header:
 // bits 0-7 the chunk's edges (kEdgeCap + 1: more than it holds), 8-20 its first
 // non-NaN sample, 21 and 22 the states of its first and last one (1: v <=
 // threshold), 23 whether it has any, 24-31 the cluster's index in its launch

@@ -194,7 +194,7 @@ struct vhsdecode_gb300_session {
     std::vector<cudaEvent_t> seg_copied, seg_dem;
     int nseg_max = 0;
     int64_t seg_cap = 0;                 // pulse events per segment
-    DevBuf<int64_t> seg_events;          // one segment's (scan of a stream with a full edge record)
+    DevBuf<int64_t> seg_events;          // one segment's (scanned behind a full edge record)
     DevBuf<unsigned> blk_counters;       // demod block claims, one counter per launch
     // pinned: kEdgePad words, max_blocks * kEdgeRecords * kEdgeWords of records,
     // nseg_max * num_sms / 2 progress words
