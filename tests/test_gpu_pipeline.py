@@ -150,3 +150,34 @@ def test_crowded_blocks_scan_their_segment(gpu, mhz, fields, crowds, segments):
             got = (s.tbc(), np.concatenate([s.lines(i) for i in range(r.fields)]))
             pictures = pictures or got
             assert all(np.array_equal(a, b) for a, b in zip(got, pictures)), source
+
+
+def test_failed_decode_leaves_nothing_behind(gpu):
+    # a segment with more edges than the host accepts (a 0.4 MHz wave for 128
+    # blocks at 20 MSPS) fails the decode while thousands of blocks are still to
+    # come; once the call has returned, nothing reads the caller's buffer any
+    # more, and a decode on another stream is what it is in a new session
+    import torch
+    from oracle import formats
+    from vhsd_gb300 import native, synth
+    clean, _ = synth.generate(synth.ntsc_vhs(fs=20e6, fields=4, seed=31, snr_db=40.0))
+    fmt = formats.get("NTSC")["sys"]
+    t = np.arange(140 * STRIDE)
+    ire = np.where((t * 0.8e6 / 20e6).astype(np.int64) % 2 == 0, -60.0, 20.0)
+    wave = 8000.0 * np.cos(2 * np.pi * np.cumsum(fmt["ire0"] + fmt["hz_ire"] * ire) / 20e6)
+    rf = np.resize(clean, 2999 * STRIDE + BLOCK)
+    rf[36 * STRIDE:36 * STRIDE + len(t)] = np.round(wave)
+    pinned = torch.from_numpy(rf).pin_memory()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with native.Session(native.PROFILE_NTSC, len(clean), sample_rate_mhz=20.0) as s:
+        s.decode(clean)
+        want = s.tbc()
+    with native.Session(native.PROFILE_NTSC, len(rf), sample_rate_mhz=20.0) as s:
+        for _ in range(3):
+            s.set_stream(first.cuda_stream)
+            with pytest.raises(native.NativeError, match="capacity"):
+                s.decode(pinned.numpy())
+            assert first.query()
+            s.set_stream(second.cuda_stream)
+            s.decode(clean)
+            assert np.array_equal(s.tbc(), want)

@@ -1381,14 +1381,12 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     s->segments = (uint32_t)nseg;
     if (nseg > s->nseg_max) throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "segment table too small");
     if (!demod_only && nseg > 0) {
-        // a demod that an earlier decode left behind (it failed) reads the tag when it starts
-        if (s->edges_pending) ck(cudaStreamSynchronize(cs), "sync");
+        // (a launch reads the tag as it starts; no earlier decode has one left, drain_session)
         if (++s->edge_tag == 0) {   // 2^32 decodes on: no word may look new
             std::memset(s->h_edges, 0, s->edge_words * sizeof(uint64_t));
             s->edge_tag = 1;
         }
         __atomic_store_n(reinterpret_cast<uint32_t*>(s->h_edges), s->edge_tag, __ATOMIC_RELEASE);
-        s->edges_pending = true;
     }
     if (graphable && nseg > 0) {
         PipeKey key{s->in_f32 ? (const void*)s->in_f32 : (const void*)rf, n, host_input, demod_only,
@@ -1446,7 +1444,6 @@ void decode_fp32_pipelined(vhsdecode_gb300_session* s, const int16_t* rf, uint64
     finish_chroma_blocks(s, cs);
     // every launch: they alternate between two streams, so the last one may end before the one ahead of it
     ck(cudaEventSynchronize(s->pipe_end), "sync");
-    s->edges_pending = false;
     demod_ms = 0.0f;
     for (int k = 0; k < nseg; k++) {
         float t = 0.0f;
@@ -1544,9 +1541,18 @@ const float* stage_float_input(vhsdecode_gb300_session* s, const void* rf, uint6
     return s->rf_f32.p;
 }
 
+// Waits for whatever a decode that failed has left on the device: it reads the
+// caller's capture and writes what the next decode writes.
+void drain_session(vhsdecode_gb300_session* s) {
+    for (cudaStream_t st : {s->stream, s->copy_stream, s->alt_stream, s->chroma_stream, s->field_stream,
+                            s->drop_stream, s->aux_stream})
+        if (st) cudaStreamSynchronize(st);
+    cudaGetLastError();   // the failure itself is the caller's
+}
+
 int32_t decode_impl(vhsdecode_gb300_session* s, const void* rf_in, uint64_t n_in, uint32_t max_fields,
                     uint32_t flags, vhsdecode_gb300_decode_result_v1* res,
-                    const std::atomic<bool>* cancel, DecodeCarry* carry) {
+                    const std::atomic<bool>* cancel, DecodeCarry* carry) try {
     if (n_in > s->max_samples)
         throw Failure(VHSDECODE_GB300_STATUS_INVALID_ARGUMENT, "sample_count exceeds the session capacity");
     ck(cudaSetDevice(s->device), "cudaSetDevice");
@@ -1630,6 +1636,9 @@ int32_t decode_impl(vhsdecode_gb300_session* s, const void* rf_in, uint64_t n_in
         res->fft_plan = (uint32_t)s->fft_plan;
     }
     return VHSDECODE_GB300_STATUS_OK;
+} catch (...) {
+    drain_session(s);
+    throw;
 }
 
 // ---------------------------------------------------------------- batched windows

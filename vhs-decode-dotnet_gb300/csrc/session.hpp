@@ -202,7 +202,6 @@ struct vhsdecode_gb300_session {
     uint64_t* h_progress = nullptr;
     size_t edge_words = 0;
     uint32_t edge_tag = 0;               // of the current decode
-    bool edges_pending = false;          // a demod that writes edges may still be running
     int rescue_fetches = 0;
     int recoveries = 0;                  // field attempts that failed and were skipped past
     uint32_t launches = 0;               // kernels started by the current decode
