@@ -181,3 +181,24 @@ def test_failed_decode_leaves_nothing_behind(gpu):
             s.set_stream(second.cuda_stream)
             s.decode(clean)
             assert np.array_equal(s.tbc(), want)
+
+
+@pytest.mark.parametrize("precision", ["FP32_FUSED", "FP64_PLAIN"])
+def test_chroma_stream_needs_no_device_memory(gpu, precision):
+    # reading the chroma channel of a decode allocates nothing on the device, so
+    # it cannot fail where the decode did not; any range of it is the part of
+    # the whole, across block ends too
+    import torch
+    from vhsd_gb300 import native, synth
+    rf, _ = synth.generate(synth.ntsc_vhs(fields=2, seed=41, snr_db=40.0))
+    rf = np.resize(rf, 199 * STRIDE + BLOCK)
+    with native.Session(native.PROFILE_NTSC, len(rf), precision=getattr(native, "PRECISION_" + precision)) as s:
+        r = s.decode(rf, chroma=True, demod_only=True)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        whole = s.stream(3, 0, r.stream_samples)
+        assert torch.cuda.mem_get_info()[0] == free
+        assert np.any(whole)
+        for start, count in ((0, 1), (STRIDE - 1, 2), (5 * STRIDE, STRIDE), (7 * STRIDE + 11, 3 * STRIDE),
+                             (r.stream_samples - 5, 5), (r.stream_samples, 0)):
+            assert np.array_equal(s.stream(3, start, count), whole[start:start + count]), (start, count)

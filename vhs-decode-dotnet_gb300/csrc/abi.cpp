@@ -476,16 +476,23 @@ void finish_chroma_blocks(vhsdecode_gb300_session* s, cudaStream_t st) {
     ck(cudaStreamWaitEvent(st, s->chroma_done, 0), "wait");
 }
 
-// The last decode's chroma channel, stitched into c32.
-void stitch_chroma(vhsdecode_gb300_session* s) {
-    if (s->c32_valid) return;
-    ck(cudaSetDevice(s->device), "cudaSetDevice");
-    const size_t want = (size_t)std::max<int64_t>(1, s->max_blocks) * kStride;
-    if (s->c32.n < want) s->c32.alloc(want);
-    ck(launch_chroma_stitch(chroma_block_params(s, nullptr, s->chroma_blocks), s->c32.p, s->chroma_stream),
-       "chroma stitch launch");
-    ck(cudaStreamSynchronize(s->chroma_stream), "sync");
-    s->c32_valid = true;
+// Samples [start, start + count) of the last decode's chroma channel (a float
+// channel in both precisions), stitched on the host from the block stage's rows
+// and means: the device holds no stitched stream.
+void copy_chroma_stream(vhsdecode_gb300_session* s, uint64_t start, uint64_t count, double* dst) {
+    if (count == 0) return;
+    const uint64_t b0 = start / kStride, nb = (start + count - 1) / kStride - b0 + 1;
+    const size_t n = (size_t)((nb - 1) * kChromaRowStride + kStride);
+    std::unique_ptr<float[]> rows(new float[n]);
+    std::vector<float> mean((size_t)nb);
+    ck(cudaMemcpy(rows.get(), s->c_scratch.p + b0 * kChromaRowStride + chroma_row_offset(s->cd.move), n * sizeof(float),
+                  cudaMemcpyDeviceToHost), "d2h");
+    ck(cudaMemcpy(mean.data(), s->c_mean.p + b0, nb * sizeof(float), cudaMemcpyDeviceToHost), "d2h");
+    for (uint64_t b = 0; b < nb; b++) {
+        const uint64_t first = std::max(start, (b0 + b) * kStride), end = std::min(start + count, (b0 + b + 1) * kStride);
+        const float* row = rows.get() + b * kChromaRowStride + (first - (b0 + b) * kStride);
+        for (uint64_t i = 0; i < end - first; i++) dst[first - start + i] = row[i] - mean[(size_t)b];
+    }
 }
 
 void session_free(vhsdecode_gb300_session* s) {
@@ -1563,7 +1570,7 @@ int32_t decode_impl(vhsdecode_gb300_session* s, const void* rf_in, uint64_t n_in
     s->want_chroma = (flags & VHSDECODE_GB300_DECODE_CHROMA) != 0;
     if (s->want_chroma) ensure_chroma(s);
     s->chroma_blocks = 0;
-    s->chroma_means = s->c32_valid = false;
+    s->chroma_means = false;
     if (!host_input && ((uintptr_t)rf_in & 15u) != 0)
         throw Failure(VHSDECODE_GB300_STATUS_INVALID_ARGUMENT, "device rf pointer must be 16-byte aligned");
     // samples at the decode rate
@@ -2028,11 +2035,8 @@ VHSDECODE_GB300_API int32_t VHSDECODE_GB300_CALL vhsdecode_gb300_session_copy_st
         uint64_t len = (uint64_t)s->last_blocks * kStride;
         if (start + count > len) return fail(VHSDECODE_GB300_STATUS_INVALID_ARGUMENT, "range beyond the stream");
         ck(cudaStreamSynchronize(s->stream), "sync");
-        if (channel == 3) {   // the chroma channel is float in both precisions
-            std::vector<float> tmp(count);
-            stitch_chroma(s);
-            ck(cudaMemcpy(tmp.data(), s->c32.p + start, count * sizeof(float), cudaMemcpyDeviceToHost), "d2h");
-            for (uint64_t i = 0; i < count; i++) dst[i] = tmp[i];
+        if (channel == 3) {
+            copy_chroma_stream(s, start, count, dst);
         } else if (s->fp32()) {
             const float* src = channel == 0 ? s->v32.p : channel == 1 ? s->s32.p : s->e32.p;
             std::vector<float> tmp(count);

@@ -13,7 +13,7 @@
 // stays in the blocks' rows, with the blocks' means beside them, and the TBC
 // takes sample s of block b as row[b][s + offset] - mean[b].  (A stitched
 // stream cost a read and a write of every sample, 0.1 ms of a 41 M-sample
-// decode's demodulation; it is made when copy_stream asks for it.)
+// decode's demodulation; copy_stream stitches on the host what it is asked for.)
 //
 // Field stage: burst probes of the line-1 chroma TBC for both rotation
 // sequences of every field (ProbeUpconvertedBurstValue + DemodBurstFloat32,
@@ -370,14 +370,6 @@ __global__ void __launch_bounds__(32) k_chroma_block_mean(ChromaBlockParams p) {
     float l8 = __fadd_rn(t, __shfl_down_sync(kFull, t, 16));
     for (int c = 8; c > 1; c /= 2) l8 = __fadd_rn(l8, __shfl_down_sync(kFull, l8, c / 2));
     if (lane == 0) p.mean[j] = __fdiv_rn(l8, (float)kBlock);
-}
-
-// The stitched channel: the kept samples of the rolled blocks minus the means.
-__global__ void __launch_bounds__(256) k_chroma_block_stitch(ChromaBlockParams p, float* out) {
-    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, j = at / kStride;
-    const int s = (int)(at - j * kStride);
-    const float* y = p.scratch + j * (int64_t)kChromaRowStride + chroma_row_offset(p.move);
-    out[at] = __fsub_rn(y[s], p.mean[j]);
 }
 
 // ---------------------------------------------------------------- burst probes
@@ -1056,13 +1048,6 @@ cudaError_t launch_chroma_blocks(const ChromaBlockParams& p, cudaStream_t s) {
 cudaError_t launch_chroma_means(const ChromaBlockParams& p, cudaStream_t s) {
     if (p.nblocks <= 0) return cudaSuccess;
     k_chroma_block_mean<<<(unsigned)p.nblocks, 32, 0, s>>>(p);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_chroma_stitch(const ChromaBlockParams& p, float* out, cudaStream_t s) {
-    if (p.nblocks <= 0) return cudaSuccess;
-    static_assert(kStride % 256 == 0, "whole CTAs");
-    k_chroma_block_stitch<<<(unsigned)(p.nblocks * (kStride / 256)), 256, 0, s>>>(p, out);
     return cudaGetLastError();
 }
 

@@ -299,11 +299,9 @@ constexpr int kChromaBlockKernels = 2;   // band-pass, means
 cudaError_t prepare_chroma_kernels();
 // CTAs (one per SM) of the chroma block stage for nblocks blocks.
 int chroma_block_ctas(int64_t nblocks);
-// The band-pass into the rows; the means of the complete rows; the stitched
-// channel.
+// The band-pass into the rows; the means of the complete rows.
 cudaError_t launch_chroma_blocks(const ChromaBlockParams& p, cudaStream_t stream);
 cudaError_t launch_chroma_means(const ChromaBlockParams& p, cudaStream_t stream);
-cudaError_t launch_chroma_stitch(const ChromaBlockParams& p, float* out, cudaStream_t stream);
 
 // Per-field chroma stages of a field batch (every array offset to the batch).
 struct ChromaFieldParams {

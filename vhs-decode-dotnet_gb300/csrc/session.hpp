@@ -231,10 +231,8 @@ struct vhsdecode_gb300_session {
     bool chroma_alloc = false;
     bool want_chroma = false;            // the current decode renders chroma
     vhsd::ChromaDesign cd;
-    DevBuf<float> c32;                   // stitched chroma stream (made by copy_stream)
-    bool c32_valid = false;              //   it holds the last decode's channel
     DevBuf<float> c_mean;                // means of the chroma blocks
-    DevBuf<float> c_scratch;             // block band-pass passes [max_blocks * (kBlock + 2 edge)]
+    DevBuf<float> c_scratch;             // band-passed blocks [max_blocks * kChromaRowStride]
     DevBuf<float> c_het, c_bsin, c_bcos; // field tables
     DevBuf<float> c_ana;                 // line-1 chroma TBC, probe windows
     DevBuf<float> c_field, c_up, c_fwd;  // output-line chroma TBC, up-converted / filtered, forward pass
