@@ -202,3 +202,42 @@ def test_chroma_stream_needs_no_device_memory(gpu, precision):
         for start, count in ((0, 1), (STRIDE - 1, 2), (5 * STRIDE, STRIDE), (7 * STRIDE + 11, 3 * STRIDE),
                              (r.stream_samples - 5, 5), (r.stream_samples, 0)):
             assert np.array_equal(s.stream(3, start, count), whole[start:start + count]), (start, count)
+
+
+@pytest.mark.parametrize("blocks,limit,batch", [(128, 100, 64), (64, 3, 2), (64, 1, 1)])
+def test_plain_workspace_takes_the_room_there_is(gpu, monkeypatch, blocks, limit, batch):
+    # a device without room for the plain demodulator's whole batch gets half as
+    # many blocks until they fit, down to one; the streams are the same (29
+    # kernels a batch)
+    from vhsd_gb300 import native, synth
+    rf, _ = synth.generate(synth.pal_vhs(fields=1, seed=51, snr_db=40.0, dropouts=10))
+    rf = np.resize(rf, (blocks - 1) * STRIDE + BLOCK)
+
+    def streams():
+        with native.Session(native.PROFILE_PAL, len(rf), precision=native.PRECISION_FP64_PLAIN) as s:
+            r = s.decode(rf, demod_only=True)
+            return r.kernel_launches, [s.stream(c, 0, r.stream_samples) for c in range(3)]
+
+    kernels, want = streams()
+    assert kernels == 29
+    monkeypatch.setenv("VHSD_PLAIN_BATCH_LIMIT", str(limit))
+    kernels, got = streams()
+    assert kernels == 29 * (blocks // batch)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+def test_chroma_finds_room_beside_the_plain_workspace(gpu, monkeypatch):
+    # buffers that a later decode adds (here the chroma workspace, refused beside
+    # a plain workspace of many blocks) take the room of the batches
+    from vhsd_gb300 import native, synth
+    rf, _ = synth.generate(synth.ntsc_vhs(fields=2, seed=52, snr_db=40.0))
+    kw = dict(precision=native.PRECISION_FP64_PLAIN)
+    with native.Session(native.PROFILE_NTSC, len(rf), **kw) as s:
+        s.decode(rf, chroma=True)
+        want = s.tbc(), s.chroma()
+    monkeypatch.setenv("VHSD_FORCE_CHROMA_WORKSPACE_FAILURE", "batched")
+    with native.Session(native.PROFILE_NTSC, len(rf), **kw) as s:
+        s.decode(rf)
+        s.decode(rf, chroma=True)
+        assert all(np.array_equal(a, b) for a, b in zip((s.tbc(), s.chroma()), want))

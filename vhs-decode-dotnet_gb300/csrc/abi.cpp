@@ -116,6 +116,36 @@ void resolve_span(int64_t intended, int64_t read_len, int64_t& s0, int64_t& slen
 FastDemodParams fp32_params(vhsdecode_gb300_session* s, const int16_t* rf_dev);
 int tuned_fft_plan(vhsdecode_gb300_session* s, FastDemodParams base);
 
+// The plain demodulator's workspace: `batch` blocks (2.5 MB each) or, where the
+// device has no room for them, half as many until it has (VHSD_PLAIN_BATCH_LIMIT:
+// no room for more, for tests).  Results do not depend on the batch.
+void alloc_plain(vhsdecode_gb300_session* s, int64_t batch) {
+    const char* limit = std::getenv("VHSD_PLAIN_BATCH_LIMIT");
+    for (;; batch /= 2) {
+        try {
+            s->plain_batch = 0;
+            s->pwork.alloc(3 * (size_t)batch * kBlock);
+            s->pdwork.alloc(3 * (size_t)batch * kBlock);
+            s->pfwork.alloc((size_t)batch * kBlock);
+            s->pflag.alloc((size_t)batch);
+            s->pmask.alloc((size_t)batch * (kBlock / 32));
+            if (limit && batch > std::max(1, std::atoi(limit)))
+                throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "plain workspace cudaMalloc: out of memory (forced)");
+            ck(cudaMemset(s->pflag.p, 0, (size_t)batch * sizeof(int)), "memset");
+            s->plain_batch = batch;
+            return;
+        } catch (const Failure&) {
+            cudaGetLastError();
+            s->pwork.release();
+            s->pdwork.release();
+            s->pfwork.release();
+            s->pflag.release();
+            s->pmask.release();
+            if (batch <= 1) throw;
+        }
+    }
+}
+
 void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_config_v1& c) {
     if (!format_for(c.profile, c.tape_speed, c.tape_format, s->fmt))
         throw Failure(VHSDECODE_GB300_STATUS_INVALID_ARGUMENT,
@@ -248,14 +278,7 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
             s->sub64.alloc(H);
             ck(cudaMemcpy(s->sub64.p, hv.data(), H * sizeof(double2), cudaMemcpyHostToDevice), "upload");
         }
-        const size_t batch = (size_t)std::min<int64_t>(std::max<int64_t>(1, s->max_blocks), kPlainBatch);
-        s->pwork.alloc(3 * batch * kBlock);
-        s->pdwork.alloc(3 * batch * kBlock);
-        s->pfwork.alloc(batch * kBlock);
-        s->pflag.alloc(batch);
-        s->pmask.alloc(batch * (kBlock / 32));
         s->ptwiddle.alloc(kBlock);
-        ck(cudaMemset(s->pflag.p, 0, batch * sizeof(int)), "memset");
         ck(make_fp64_twiddles(s->ptwiddle.p, s->own_stream), "twiddles");
         ck(cudaStreamSynchronize(s->own_stream), "sync");
     }
@@ -343,6 +366,21 @@ void session_init(vhsdecode_gb300_session* s, const vhsdecode_gb300_session_conf
     s->drop_out.alloc((size_t)s->max_fields * s->drop_out_cap * 3);
     s->drop_out_count.alloc(s->max_fields);
     s->drop_status.alloc(s->max_fields);
+    if (!s->fp32()) alloc_plain(s, std::min<int64_t>(std::max<int64_t>(1, s->max_blocks), kPlainBatch));
+}
+
+// Runs an allocation; where it finds no room beside a plain workspace of many
+// blocks, once more beside one of a single block.
+template <typename F>
+void with_room(vhsdecode_gb300_session* s, F alloc) {
+    try {
+        alloc();
+    } catch (const Failure&) {
+        if (s->plain_batch <= 1) throw;
+        cudaGetLastError();
+        alloc_plain(s, 1);
+        alloc();
+    }
 }
 
 // Chroma tables and buffers, made by the first decode that renders chroma.
@@ -367,7 +405,9 @@ void ensure_chroma(vhsdecode_gb300_session* s) {
     // tools/build-cuda-fast-native.ps1:290-305): the workspace allocation
     // fails partway, and the decode must fail rather than report chroma it
     // never wrote.  A later call allocates the workspace afresh.
-    if (const char* f = std::getenv("VHSD_FORCE_CHROMA_WORKSPACE_FAILURE"); f && *f && std::strcmp(f, "0") != 0)
+    // ("batched": only beside a plain workspace of more than one block.)
+    if (const char* f = std::getenv("VHSD_FORCE_CHROMA_WORKSPACE_FAILURE");
+        f && *f && std::strcmp(f, "0") != 0 && (std::strcmp(f, "batched") != 0 || s->plain_batch > 1))
         throw Failure(VHSDECODE_GB300_STATUS_INTERNAL_ERROR, "chroma workspace cudaMalloc: out of memory (forced)");
     std::vector<float> het, bsin, bcos;
     vhsd::chroma_tables(d, het, bsin, bcos);
@@ -682,6 +722,7 @@ void run_demod(vhsdecode_gb300_session* s, const int16_t* rf_dev, int64_t nblock
         ck(cudaMemsetAsync(s->repair.p, 0, sizeof(int), s->stream), "memset");
         ck(launch_fused(s, p, s->stream), "demod fp32 launch");
     } else {
+        if (s->plain_batch == 0) alloc_plain(s, 1);   // an earlier decode found no room at all
         PlainDemodParams p{};
         p.rf = s->in_f32 ? nullptr : rf_dev;
         p.rf_f32 = s->in_f32;
@@ -707,7 +748,7 @@ void run_demod(vhsdecode_gb300_session* s, const int16_t* rf_dev, int64_t nblock
             p.sub.high = s->sub64.p;
         }
         // batches of equal size
-        const int64_t batches = (nblocks + kPlainBatch - 1) / kPlainBatch;
+        const int64_t batches = (nblocks + s->plain_batch - 1) / s->plain_batch;
         for (int64_t k = 0; k < batches; k++) {
             p.first_block = nblocks * k / batches;
             p.nblocks = (int)(nblocks * (k + 1) / batches - p.first_block);
@@ -1512,7 +1553,7 @@ const float* stage_float_input(vhsdecode_gb300_session* s, const void* rf, uint6
     cudaStream_t cs = s->stream;
     const uint64_t nd = n / (uint64_t)s->decim;
     auto ensure = [&](DevBuf<float>& b, uint64_t count) {
-        if (b.n < count) b.alloc(count);
+        if (b.n < count) with_room(s, [&] { b.alloc(count); });
     };
     if (s->decim == 1) {   // float input at the decode rate
         if (!host_input) return static_cast<const float*>(rf);
@@ -1568,7 +1609,7 @@ int32_t decode_impl(vhsdecode_gb300_session* s, const void* rf_in, uint64_t n_in
     const bool demod_only = (flags & VHSDECODE_GB300_DECODE_DEMOD_ONLY) != 0;
     const bool f32_in = (flags & VHSDECODE_GB300_DECODE_FLOAT_INPUT) != 0;
     s->want_chroma = (flags & VHSDECODE_GB300_DECODE_CHROMA) != 0;
-    if (s->want_chroma) ensure_chroma(s);
+    if (s->want_chroma) with_room(s, [&] { ensure_chroma(s); });
     s->chroma_blocks = 0;
     s->chroma_means = false;
     if (!host_input && ((uintptr_t)rf_in & 15u) != 0)

@@ -158,6 +158,7 @@ struct vhsdecode_gb300_session {
     DevBuf<double2> vid64, syn64, sub64;
     DevBuf<float2> scratch;
     DevBuf<int> repair;
+    int64_t plain_batch = 0;             // blocks that its workspace holds
     DevBuf<double2> pwork;
     DevBuf<double> pdwork;
     DevBuf<float> pfwork;
