@@ -1176,11 +1176,15 @@ void collect_field_results(vhsdecode_gb300_session* s, cudaStream_t fs) {
 
 // Segment boundaries (in blocks) of the pipelined decode: a short first
 // segment so the demod can start soon behind its RF copy, then kSegBlocks each;
-// `growing`, each after the first twice as long as the one before: pinned
-// memory is copied at more than twice the demodulator's rate, and each launch
-// costs its clusters a start (60 NTSC fields, luma, 12 launches 2.03 ms, 5
-// launches 2.00; 120 fields, 22 and 6, 3.75 and 3.66).  Pageable memory is
-// copied at about the demodulator's rate, so there the steps stay short.
+// `growing` (a pinned capture whose launches are replayed from a graph), each
+// after the first twice as long as the one before: pinned memory is copied at
+// more than twice the demodulator's rate, and each launch costs its clusters a
+// start (60 NTSC fields, luma, 12 launches 2.03 ms, 5 launches 2.00; 120
+// fields, 22 and 6, 3.75 and 3.66).  Pageable memory is copied at about the
+// demodulator's rate, so there the steps stay short.  The windows of run() and
+// the server are pinned, are not replayed, and keep the short steps too: with
+// growing ones four windows at once took 3.67 to 3.69 ms against 3.70, a
+// 12-field run 16.3 against 15.9 to 16.1, both within the runs' difference.
 std::vector<int64_t> segment_bounds(int64_t nblocks, bool growing = false) {
     std::vector<int64_t> b{0};
     int64_t e = std::min<int64_t>(nblocks, kFirstSegBlocks), step = kSegBlocks;

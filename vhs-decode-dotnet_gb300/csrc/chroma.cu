@@ -211,7 +211,7 @@ __device__ __forceinline__ void iir_compute(const float (&sec)[6], float z1, flo
     }
 }
 
-// Lane `h` (0 .. 3) of a block's group in a helper warp: an eighth of every
+// Lane `h` (0 .. 3) of a block's group in a helper warp: its quarter of every
 // chunk is 16 bytes of int16 source, 32 bytes of floats.  kMode 0: forward
 // over the int16 block, 1: forward over the float block, 2: backward over the
 // forward output.  The forward pass writes sample e at row[5 + e]; the

@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(kPT) k_pulse_bits(const unsigned* __restrict__
 // through distributed shared memory, over the cluster, writes its events.
 // Edges alternate, so an event's type follows from the state entering its word
 // and its place in it.  What bounds a short scan is launches: the two passes
-// and the ticket's memset took 15 us a call for 65,536 samples, this 11.
+// and the ticket's memset took 14.9 us a call for 65,536 samples, this 10.0
+// (9.3 to 10.9 in six runs).
 template <typename T>
 __global__ void __launch_bounds__(1024) k_pulse_cluster(const T* __restrict__ ref, int64_t begin, int64_t end, Cmp<T> cmp,
                                                         int64_t* events, int64_t capacity, int64_t* total) {
@@ -1520,8 +1521,7 @@ __device__ __forceinline__ void tap_sums(const float (&x)[16], const float (&y)[
 // shared-memory / L1 data path: 128 bytes of the sinc LUT at a random row and
 // 16 (with kPair 32) source floats per sample.  So:
 // * the line's stretch of the source is staged in shared memory once, and a
-//   lane reads its 16 floats with nine 8-byte loads (4 wavefronts a warp each;
-//   from global memory, 8 bytes a lane, 7);
+//   lane reads its 16 floats with five 16-byte loads (load_taps);
 // * a warp fetches its 32 samples' LUT rows together, a quad of lanes per
 //   sample and 32 bytes a lane, so a row pair is one 128-byte access; the quad
 //   interpolates and leaves the 16 weights in the sample's shared row;
